@@ -72,7 +72,7 @@ def units(mech: str) -> tuple[str, ...]:
 
 def _sources(mech: str) -> list[Path]:
     return [*(CSRC / u for u in units(mech)), CSRC / "capi_common.cuh", CSRC / "solver.cuh", CSRC / "eval_common.cuh",
-            CSRC / "mkpp_device.cuh", GEN / f"{mech}.cuh", INCLUDE / "mkpp.h", Path(__file__)]
+            CSRC / "mkpp_device.cuh", CSRC / "warp_engine.cuh", GEN / f"{mech}.cuh", INCLUDE / "mkpp.h", Path(__file__)]
 
 
 def _stale(mech: str) -> bool:

@@ -65,9 +65,10 @@ int launch_fixed_columns(size_t n, const double* conc, const double* temp, const
                          const double* clw, const double* param, double* out, cudaStream_t stream);
 // mkpp_plain.cu: the grid-stride integrate (255-register variant).
 int launch_plain(const mkpp::LaunchArgs& a, double* scratch, int grid, cudaStream_t stream);
-// mkpp_coop.cu: the warp-cooperative integrate of parked cells.
-int set_coop_smem(size_t bytes);
-int launch_coop(const mkpp::LaunchArgs& a, int grid, int threads, size_t smem, cudaStream_t stream);
+// mkpp_coop.cu: the warp-cooperative integrate (one warp per block, `smem`
+// bytes each) and its blocks per SM (0: it cannot run).
+int coop_resident_blocks(size_t smem);
+int launch_coop(const mkpp::LaunchArgs& a, int grid, size_t smem, cudaStream_t stream);
 // ... and the split form (integrate_split_kernel: whole warps on reserved
 // SMs, the persistent body on the others).
 int launch_split(const mkpp::LaunchArgs& a, double* scratch, int grid, cudaStream_t stream);

@@ -114,7 +114,7 @@ int device_fail(mkpp_handle_s* h, cudaError_t err, const char* what) {
 //                    persistent kernel parks a cell for the warp-cooperative
 //                    kernel (0: never).  A launch over S host steps parks a
 //                    cell after defer_after * S attempts in all.  A
-//                    cooperative SAPRC99 attempt takes ~0.37 ms against
+//                    cooperative SAPRC99 attempt takes ~0.19 ms against
 //                    ~1 ms on one lane, but the cooperative kernel has about
 //                    a fifth of the lanes' throughput, so only the tail
 //                    should park.  The default, 3000, parks ~7% of the cells
@@ -139,6 +139,16 @@ struct Tuning {
   // persistent body runs on the others (0: off).
   int split_cells = 0;
   int split_sms = 0;
+  // Calls of at most this many cells run on the cooperative kernel alone
+  // (coop_alone).  A lane needs 1.0 ms for a SAPRC99 attempt
+  // and 1.9 ms with every SM full, a warp 0.19 ms; with eight warps per SM the
+  // warps reach 5.2 M attempts/s against the lanes' 2.9 M in one host step of
+  // 32768 cells (206 against 371 ms; 2500 cells: 34 against 163 ms), and the
+  // lanes' 6.2 M in four host steps of 65536.  A table-driven mechanism (TS1)
+  // is always faster there: 79 against 293 ms for 4096 cells.  A mechanism
+  // with few operations per attempt spends them on the parts that every lane
+  // of the warp repeats, so it stays on lanes.
+  int coop_cells = Mech::TABLE_ATTEMPT ? INT32_MAX : Mech::LU_FMA > 2000 ? 40000 : 0;
 };
 
 Tuning& tuning() {
@@ -148,6 +158,7 @@ Tuning& tuning() {
     if (const char* e = std::getenv("MKPP_BLOCKS_PER_SM")) x.blocks_per_sm = std::max(0, std::atoi(e));
     if (const char* e = std::getenv("MKPP_DEFER_AFTER")) x.defer_after = std::max(0, std::atoi(e));
     if (const char* e = std::getenv("MKPP_TAIL_AFTER")) x.tail_after = std::max(0, std::atoi(e));
+    if (const char* e = std::getenv("MKPP_COOP_CELLS")) x.coop_cells = std::max(0, std::atoi(e));
     return x;
   }();
   return t;
@@ -157,9 +168,7 @@ struct LaunchConfig {
   int minb = 0;
   int grid = 0;
   int sms = 0;
-  int coop_warps = 0;
-  size_t coop_smem = 0;
-  bool coop_ok = false;
+  int coop_per_sm = 0;  // cooperative warps per SM (0: no cooperative kernel)
   bool split_ok = false;
 };
 
@@ -169,6 +178,8 @@ int resident_blocks() {
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mkpp::integrate_persistent_kernel<Mech, MINB>, mkpp::kBlock, 0);
   return std::max(1, per_sm);
 }
+
+constexpr size_t kCoopSmem = (size_t)Mech::COOP_SLOTS * sizeof(double);
 
 LaunchConfig g_config;
 
@@ -184,13 +195,9 @@ const LaunchConfig& launch_config() {
     int per_sm = cfg.minb == 4 ? resident_blocks4() : resident_blocks<2>();
     if (t.blocks_per_sm > 0) per_sm = std::min(per_sm, t.blocks_per_sm);
     cfg.grid = cfg.sms * per_sm;
-    // Cooperative kernel: as many warps per block (at most kCoopWarps) as fit
-    // in 200 KB of shared memory.  A cell store larger than that leaves the
-    // cooperative kernel unused (no parking).
-    const size_t per_warp = (size_t)Mech::COOP_SLOTS * sizeof(double);
-    cfg.coop_warps = (int)std::min<size_t>(mkpp::kCoopWarps, (200u * 1024u) / per_warp);
-    cfg.coop_smem = per_warp * (size_t)std::max(1, cfg.coop_warps);
-    cfg.coop_ok = cfg.coop_warps >= 1 && set_coop_smem(cfg.coop_smem) == MKPP_SUCCESS;
+    // A cell store larger than a block's shared memory leaves the cooperative
+    // kernel unused (no parking).
+    cfg.coop_per_sm = coop_resident_blocks(kCoopSmem);
     cfg.split_ok = StoreInfo::kTile;
   }
   return cfg;
@@ -198,7 +205,7 @@ const LaunchConfig& launch_config() {
 
 int integrate_grid() { return launch_config().grid; }
 
-// Workspace layout: [queue counter, parked-cell counter, active-cell counter | 256 B]
+// Workspace layout: [counters: queue, parked cells, active cells, split, cooperative | 256 B]
 // [per-block scratch tiles][parked-cell records, one per cell].
 size_t scratch_offset() { return kQueueBytes; }
 size_t defer_offset() {
@@ -224,6 +231,14 @@ int launch_rates(size_t cells, const double* conc, const double* temp, const dou
   return cudaGetLastError() == cudaSuccess ? MKPP_SUCCESS : MKPP_ERROR_DEVICE;
 }
 
+// Whether the cooperative kernel takes the whole call: few enough cells, and
+// no launch form of the persistent kernel asked for.
+bool coop_alone(const mkpp::LaunchArgs& a) {
+  const Tuning& t = tuning();
+  return a.ncells <= t.coop_cells && t.defer_after > 0 && t.register_variant == 2 && t.blocks_per_sm == 0 &&
+         !(t.split_cells > 0 && a.order);
+}
+
 int launch_integrate(const mkpp::LaunchArgs& args, int mode, void* workspace, cudaStream_t stream) {
   mkpp::LaunchArgs a = args;
   unsigned char* ws = (unsigned char*)workspace;
@@ -232,7 +247,13 @@ int launch_integrate(const mkpp::LaunchArgs& args, int mode, void* workspace, cu
   a.active = (unsigned int*)ws + 2;
   double* scratch = StoreInfo::block_bytes ? (double*)(ws + scratch_offset()) : nullptr;
   const LaunchConfig& cfg = launch_config();
-  if (cudaMemsetAsync(ws, 0, 4 * sizeof(unsigned int), stream) != cudaSuccess) return MKPP_ERROR_DEVICE;
+  a.coop_next = (unsigned int*)ws + 4;
+  if (cudaMemsetAsync(ws, 0, 5 * sizeof(unsigned int), stream) != cudaSuccess) return MKPP_ERROR_DEVICE;
+  const int coop_blocks = cfg.sms * cfg.coop_per_sm;
+  if (mode == 1 && coop_blocks > 0 && coop_alone(a)) {
+    a.coop_all = 1;
+    return launch_coop(a, std::min(a.ncells, coop_blocks), kCoopSmem, stream);
+  }
   if (mode == 1) {
     const Tuning& t = tuning();
     // Split launch: the order's first cells on whole warps on reserved SMs,
@@ -249,11 +270,11 @@ int launch_integrate(const mkpp::LaunchArgs& args, int mode, void* workspace, cu
     a.defer_after = (int)std::min<long long>(park, INT32_MAX);
     // Tail parking runs in the 255-register variant only.
     const bool tail = t.tail_after > 0 && cfg.minb == 2;
-    a.defer = (a.defer_after > 0 || tail) && cfg.coop_ok ? (mkpp::Deferred*)(ws + defer_offset()) : nullptr;
+    a.defer = (a.defer_after > 0 || tail) && coop_blocks > 0 ? (mkpp::Deferred*)(ws + defer_offset()) : nullptr;
     if (!a.defer) a.defer_after = 0;
     if (tail && a.defer) {
       a.tail_after = t.tail_after;
-      a.tail_cells = (unsigned)(cfg.sms * 2 * cfg.coop_warps);
+      a.tail_cells = (unsigned)coop_blocks;
       if (launch_persistent_tail(a, scratch, cfg.grid, stream) != MKPP_SUCCESS) return MKPP_ERROR_DEVICE;
     } else if (split) {
       if (launch_split(a, scratch, cfg.grid, stream) != MKPP_SUCCESS) return MKPP_ERROR_DEVICE;
@@ -263,7 +284,7 @@ int launch_integrate(const mkpp::LaunchArgs& args, int mode, void* workspace, cu
       mkpp::integrate_persistent_kernel<Mech, 2><<<cfg.grid, mkpp::kBlock, 0, stream>>>(a, scratch);
     }
     if (a.defer) {
-      if (launch_coop(a, cfg.sms * 2, cfg.coop_warps * 32, cfg.coop_smem, stream) != MKPP_SUCCESS) {
+      if (launch_coop(a, coop_blocks, kCoopSmem, stream) != MKPP_SUCCESS) {
         return MKPP_ERROR_DEVICE;
       }
     }

@@ -5,15 +5,18 @@
 
 namespace mkpp_tu {
 
-int set_coop_smem(size_t bytes) {
-  return cudaFuncSetAttribute(mkpp::integrate_coop_kernel<Mech>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)bytes) == cudaSuccess
-             ? MKPP_SUCCESS
-             : MKPP_ERROR_DEVICE;
+int coop_resident_blocks(size_t smem) {
+  int per_sm = 0;
+  if (cudaFuncSetAttribute(mkpp::integrate_coop_kernel<Mech>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)smem) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mkpp::integrate_coop_kernel<Mech>, 32, smem) !=
+          cudaSuccess)
+    return 0;
+  return per_sm;
 }
 
-int launch_coop(const mkpp::LaunchArgs& a, int grid, int threads, size_t smem, cudaStream_t stream) {
-  mkpp::integrate_coop_kernel<Mech><<<grid, threads, smem, stream>>>(a);
+int launch_coop(const mkpp::LaunchArgs& a, int grid, size_t smem, cudaStream_t stream) {
+  mkpp::integrate_coop_kernel<Mech><<<grid, 32, smem, stream>>>(a);
   return cudaGetLastError() == cudaSuccess ? MKPP_SUCCESS : MKPP_ERROR_DEVICE;
 }
 

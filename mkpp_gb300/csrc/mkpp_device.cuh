@@ -56,4 +56,51 @@ struct KLocal {
 
 __device__ __forceinline__ bool finite(double x) { return isfinite(x); }
 
+// ---------------------------------------------------------------------------
+// Programs of uniform operations S[out] = fma(+-S[a], S[b], S[c]) or
+// S[out] = 1 / S[b], one 64-bit word each, four 16-bit fields of slot * 4 plus
+// two flags (emitter/warp_schedule.py):
+//   a: 1 negate the product | b, c: 1 the lane's previous result instead |
+//   out: 1 store nothing, 2 reciprocal.
+// ---------------------------------------------------------------------------
+struct ProgramWord {
+  unsigned lo, hi;
+  __device__ __forceinline__ ProgramWord(unsigned long long w) : lo((unsigned)w), hi((unsigned)(w >> 32)) {}
+  __device__ __forceinline__ unsigned negate() const { return lo << 31; }  // the sign bit
+  __device__ __forceinline__ bool prev_b() const { return lo & 0x10000u; }
+  __device__ __forceinline__ bool prev_c() const { return hi & 1u; }
+  __device__ __forceinline__ bool stores() const { return !(hi & 0x10000u); }
+  __device__ __forceinline__ bool reciprocal() const { return hi & 0x20000u; }
+  __device__ __forceinline__ unsigned a() const { return (lo >> 2) & 0x3fffu; }
+  __device__ __forceinline__ unsigned b() const { return lo >> 18; }
+  __device__ __forceinline__ unsigned c() const { return (hi >> 2) & 0x3fffu; }
+  __device__ __forceinline__ unsigned out() const { return hi >> 18; }
+};
+
+__device__ __forceinline__ double flip_sign(double x, unsigned sign) {
+  return __longlong_as_double(__double_as_longlong(x) ^ ((long long)sign << 32));
+}
+__device__ __forceinline__ bool is_zero(double x) { return (__double_as_longlong(x) << 1) == 0; }
+
+// Sequential form: one thread runs `ops` words on its own store.  Returns
+// false if a reciprocal met a zero.
+template <class SA>
+__device__ __forceinline__ bool run_program(SA& S, const unsigned long long* __restrict__ prog, int ops) {
+  double prev = 0.0;
+  bool ok = true;
+  for (int n = 0; n < ops; ++n) {
+    const ProgramWord w(__ldg(prog + n));
+    const double B = w.prev_b() ? prev : S[w.b()];
+    if (w.reciprocal()) {
+      ok = ok && !is_zero(B);
+      prev = 1.0 / B;
+    } else {
+      const double C = w.prev_c() ? prev : S[w.c()];
+      prev = fma(flip_sign(S[w.a()], w.negate()), B, C);
+    }
+    if (w.stores()) S[w.out()] = prev;
+  }
+  return ok;
+}
+
 }  // namespace mkpp

@@ -18,6 +18,7 @@
 #include <type_traits>
 
 #include "mkpp_device.cuh"
+#include "warp_engine.cuh"
 
 namespace mkpp {
 
@@ -68,6 +69,10 @@ struct LaunchArgs {
   int split_cells;
   int split_sms;
   unsigned int* split_next;
+  // Cooperative kernel: its work counter (zeroed before launch), and whether
+  // it integrates every cell from its start instead of the parked ones.
+  unsigned int* coop_next;
+  int coop_all;
 };
 
 // Controller state of a parked cell (see LaunchArgs::defer).
@@ -472,14 +477,14 @@ __global__ void __launch_bounds__(kBlock, MINB) integrate_persistent_kernel(Laun
 
 
 // ---------------------------------------------------------------------------
-// Cooperative form for parked cells: a whole warp integrates one cell at a
-// time, the cell's working set in shared memory, each attempt spread over
-// the lanes by the level schedules of Mech::attempt_coop.  It resumes the
-// parked controller state exactly, and attempt_coop reproduces attempt's
-// arithmetic, so a parked cell ends bit-identical to an unparked one.
+// Cooperative form: a whole warp integrates one cell at a time, the cell's
+// working set in shared memory, each attempt spread over the lanes by the
+// program of Mech::attempt_coop.  It takes the parked cells, resuming the
+// parked controller state exactly, or (coop_all) every cell of a small call.
+// attempt_coop reproduces attempt's arithmetic, so a cell ends bit-identical
+// on either form.  A block is one warp, so that a few cells spread over the
+// SMs, and its cells come from a work counter.
 // ---------------------------------------------------------------------------
-constexpr int kCoopWarps = 4;
-
 // One cell on a whole warp, from the controller state ctl at host step
 // `step` (attempt and accept counts so far in nacc, nrej) to the end of its
 // last host step; the cell's state is in S[Y..] already.  Writes the state,
@@ -493,7 +498,6 @@ __device__ __forceinline__ void coop_integrate_cell(const LaunchArgs& a, double*
   for (; step < a.steps;) {
     for (int r = lane; r < Mech::NR; r += 32) S[Mech::KT + r] = a.ktab[(size_t)step * a.k_step_stride + c + n * r];
     __syncwarp();
-    auto k = [&](int r) { return S[Mech::KT + r]; };
     while (ctl.running()) {
       if (ctl.attempts >= a.max_attempts) {
         capped = true;
@@ -501,7 +505,7 @@ __device__ __forceinline__ void coop_integrate_cell(const LaunchArgs& a, double*
       }
       const double h = ctl.next_h();
       int st = 0;
-      const double err = Mech::attempt_coop(S, k, h, st, lane);
+      const double err = Mech::attempt_coop(S, h, st, lane, WarpProgram());
       zero_pivot |= st != 0;
       if (ctl.update<Mech>(err)) {
         for (int i = lane; i < Mech::NV; i += 32) S[Mech::Y + i] += S[Mech::DY + i];
@@ -531,29 +535,52 @@ __device__ __forceinline__ void coop_integrate_cell(const LaunchArgs& a, double*
 }
 
 template <class Mech>
-__global__ void __launch_bounds__(kCoopWarps * 32, 1) integrate_coop_kernel(LaunchArgs a) {
+__global__ void __launch_bounds__(32) integrate_coop_kernel(LaunchArgs a) {
   extern __shared__ double smem[];
-  const unsigned lane = threadIdx.x & 31u;
-  const unsigned wib = threadIdx.x >> 5;
-  const unsigned wpb = blockDim.x >> 5;  // warps launched per block (<= kCoopWarps)
-  double* S = smem + (size_t)wib * Mech::COOP_SLOTS;
+  const unsigned lane = threadIdx.x;
+  double* S = smem;
   const size_t n = (size_t)a.ncells;
-  const unsigned count = *a.defer_count;
-  for (unsigned idx = blockIdx.x * wpb + wib; idx < count; idx += gridDim.x * wpb) {
-    const Deferred d = a.defer[idx];
-    const size_t c = (size_t)d.cell;
+  const unsigned count = a.coop_all ? (unsigned)a.ncells : *a.defer_count;
+  Mech::coop_constants(S, lane);
+  // Every pass takes a new counter value, so a warp makes at most count + 1
+  // passes.
+  for (unsigned pass = 0; pass <= count; ++pass) {
+    unsigned idx = 0;
+    if (lane == 0) idx = atomicAdd(a.coop_next, 1u);
+    idx = __shfl_sync(0xffffffffu, idx, 0);
+    if (idx >= count) break;
+    Controller ctl;
+    size_t c;
+    int step = 0, nacc = 0, nrej = 0;
+    bool zero_pivot = false;
+    if (a.coop_all) {
+      const long long cell = a.order ? a.order[idx] : (long long)idx;
+      if (cell < 0 || cell >= (long long)n) continue;  // an order entry out of range names no cell
+      c = (size_t)cell;
+      if (a.status && a.status[c] != CELL_SUCCESS) {
+        if (lane == 0) clear_counts(a, c);
+        continue;
+      }
+      ctl.start(a.dt, a.seed, a.dt_carry ? a.dt_carry[c] : 0.0);
+    } else {
+      const Deferred d = a.defer[idx];
+      c = (size_t)d.cell;
+      ctl.start(a.dt, a.seed);
+      ctl.t = d.t;
+      ctl.dt = d.dt;
+      ctl.want = d.want;
+      ctl.attempts = d.attempts;
+      ctl.reject_last = d.flags & 1;
+      ctl.reject_more = (d.flags & 2) != 0;
+      ctl.cut = (d.flags & 8) != 0;
+      step = d.step;
+      nacc = d.nacc;
+      nrej = d.nrej;
+      zero_pivot = (d.flags & 4) != 0;
+    }
     for (int i = lane; i < Mech::NV; i += 32) S[Mech::Y + i] = a.conc[c + n * Mech::var_phys(i)];
     __syncwarp();
-    Controller ctl;
-    ctl.start(a.dt, a.seed);
-    ctl.t = d.t;
-    ctl.dt = d.dt;
-    ctl.want = d.want;
-    ctl.attempts = d.attempts;
-    ctl.reject_last = d.flags & 1;
-    ctl.reject_more = (d.flags & 2) != 0;
-    ctl.cut = (d.flags & 8) != 0;
-    coop_integrate_cell<Mech>(a, S, lane, c, ctl, d.step, d.nacc, d.nrej, (d.flags & 4) != 0);
+    coop_integrate_cell<Mech>(a, S, lane, c, ctl, step, nacc, nrej, zero_pivot);
   }
 }
 
@@ -573,8 +600,8 @@ __global__ void __launch_bounds__(kCoopWarps * 32, 1) integrate_coop_kernel(Laun
 // ---------------------------------------------------------------------------
 template <class Mech>
 __global__ void __launch_bounds__(kBlock, 2) integrate_split_kernel(LaunchArgs a, double* scratch) {
-  static_assert(kCoopWarps * 32 == kBlock, "a split block is kCoopWarps warps");
-  static_assert((size_t)kCoopWarps * Mech::COOP_SLOTS <= StoreFor<Mech>::block_bytes / sizeof(double),
+  constexpr int kWarps = kBlock / 32;
+  static_assert((size_t)kWarps * Mech::COOP_SLOTS <= StoreFor<Mech>::block_bytes / sizeof(double),
                 "the warps' stores fit in the block's scratch tile");
   unsigned smid;
   asm("mov.u32 %0, %%smid;" : "=r"(smid));  // the SM this block runs on
@@ -585,6 +612,7 @@ __global__ void __launch_bounds__(kBlock, 2) integrate_split_kernel(LaunchArgs a
   const unsigned lane = threadIdx.x & 31u;
   double* S = scratch + (size_t)blockIdx.x * Mech::NSLOTS * kBlock + (size_t)(threadIdx.x >> 5) * Mech::COOP_SLOTS;
   const size_t n = (size_t)a.ncells;
+  Mech::coop_constants(S, lane);
   // Every pass takes a new counter value, so a warp makes at most
   // split_cells + 1 passes.
   for (int pass = 0; pass <= a.split_cells; ++pass) {

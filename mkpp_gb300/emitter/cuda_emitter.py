@@ -128,7 +128,7 @@ def _c_array(c, ctype, name, values):
 def _c_u64_array(c, name, values):
     vals = list(values) or [0]
     rows = [", ".join(f"0x{v:x}ull" for v in vals[i:i + 8]) for i in range(0, len(vals), 8)]
-    c(f"static __device__ const unsigned long long {name}[{len(vals)}] = {{")
+    c(f"alignas(16) static __device__ const unsigned long long {name}[{len(vals)}] = {{")
     for r in rows:
         c(f"    {r},")
     c("};")
@@ -282,7 +282,13 @@ def _coop_build(plan, nv, stages, A, C, NewF, K0, Y, FS, DY, nslots, table=False
                     P.fma(kb + i, cterm_slot[(st, j)], K0 + (j - 1) * nv + i, kb + i)
         P.solve(plan, kb)
         progs.append(P.ops)
-    sched = [warp_schedule.schedule(ops) for ops in progs]
+    sched = [warp_schedule.pipeline(ops) for ops in progs]
+    # An idle step or two end each stage, so that the next one's first step
+    # finds every result in its slot and steps pair up; the last stage fills
+    # up the device loop's groups of steps.
+    for st in sched:
+        st += [[]] * (2 - len(st) % 2)
+    sched[-1] += [[]] * (-sum(map(len, sched)) % warp_schedule.AHEAD)
     adj_ops = eval_ops = None
     if table:
         P = program()
@@ -297,7 +303,8 @@ def _coop_build(plan, nv, stages, A, C, NewF, K0, Y, FS, DY, nslots, table=False
         assert all(op[0] != warp_schedule.RCP for op in eval_ops)
     nconst = 4 + len(cterm_slot) + len(literals)
     const_vals = ["-0.0", "0.0", "1.0", "0.0"] + ["0.0"] * len(cterm_slot) + [_lit(v) for v in literals]
-    return {"progs": progs, "sched": sched, "npart": npart, "nq": nq, "Q": Q, "D": D, "CB": CB,
+    seq_ops = [op for ops in progs for op in ops] if table else None
+    return {"progs": progs, "sched": sched, "seq_ops": seq_ops, "npart": npart, "nq": nq, "Q": Q, "D": D, "CB": CB,
             "nconst": nconst, "const_vals": const_vals, "literals": literals, "cterm_slot": cterm_slot,
             "KT": Mech_KT, "total": CB + nconst, "adj": adj, "adj_ops": adj_ops, "eval_ops": eval_ops,
             "A": A, "NewF": NewF}
@@ -628,13 +635,7 @@ def _emit_tlm(c, t, tlm, C):
     for (st, j), slot in tlm["cterm"].items():
         cv = C[(st - 1) * (st - 2) // 2 + j - 1]
         c(f"    S[{slot}] = {_lit(cv)} / h;    // c{st}{j} / h")
-    c("    for (int n = 0; n < coop::TLM_OPS; ++n) {")
-    c("      const unsigned long long w = __ldg(coop::tlm_prog + n);")
-    c("      const unsigned lo = (unsigned)w, hi = (unsigned)(w >> 32);")
-    c("      const double a = __longlong_as_double(__double_as_longlong(S[(lo >> 16) & 0x7fffu]) ^")
-    c("                                            ((long long)(lo >> 31) << 63));")
-    c("      S[lo & 0xffffu] = fma(a, S[hi & 0xffffu], S[(hi >> 16) & 0x7fffu]);")
-    c("    }")
+    c("    mkpp::run_program(S, coop::tlm_prog, coop::TLM_OPS);")
     c("  }")
 
 
@@ -657,13 +658,7 @@ def _emit_table_adjoint(c, coop):
     c("  __device__ __forceinline__ static void adjoint_step(SA& S, const KA& k, double h) {")
     c("    (void)k;")
     c("    (void)h;")
-    c("    for (int n = 0; n < coop::ADJ_OPS; ++n) {")
-    c("      const unsigned long long w = __ldg(coop::adj_prog + n);")
-    c("      const unsigned lo = (unsigned)w, hi = (unsigned)(w >> 32);")
-    c("      const double a = __longlong_as_double(__double_as_longlong(S[(lo >> 16) & 0x7fffu]) ^")
-    c("                                            ((long long)(lo >> 31) << 63));")
-    c("      S[lo & 0xffffu] = fma(a, S[hi & 0xffffu], S[(hi >> 16) & 0x7fffu]);")
-    c("    }")
+    c("    mkpp::run_program(S, coop::adj_prog, coop::ADJ_OPS);")
     c("  }")
     c("")
     c("  // ---- tendencies and Jacobian (table-driven evaluation entries) ----")
@@ -675,13 +670,7 @@ def _emit_table_adjoint(c, coop):
     c("    for (int r = 0; r < NR; ++r) S[KT + r] = k(r);")
     c("    for (int i = 0; i < NCONST; ++i) S[CB + i] = coop::const_val[i];")
     c("    S[CB + 3] = 0.0;  // 1/(gamma h)")
-    c("    for (int n = 0; n < coop::EVAL_OPS; ++n) {")
-    c("      const unsigned long long w = __ldg(coop::eval_prog + n);")
-    c("      const unsigned lo = (unsigned)w, hi = (unsigned)(w >> 32);")
-    c("      const double a = __longlong_as_double(__double_as_longlong(S[(lo >> 16) & 0x7fffu]) ^")
-    c("                                            ((long long)(lo >> 31) << 63));")
-    c("      S[lo & 0xffffu] = fma(a, S[hi & 0xffffu], S[(hi >> 16) & 0x7fffu]);")
-    c("    }")
+    c("    mkpp::run_program(S, coop::eval_prog, coop::EVAL_OPS);")
     c("  }")
 
 
@@ -689,12 +678,10 @@ def _emit_table_attempt_head(c, coop, C):
     """Head of the table-driven per-thread attempt (the increment and error
     norm that follow are those of the unrolled attempt)."""
     c("  // One Rosenbrock attempt of size h from the state in S[Y..], table-driven:")
-    c("  // one thread walks the stage programs of the cooperative kernel")
-    c("  // (coop::sched) on its own cell, step after step, the words of a step in")
-    c("  // order.  The operations of a step are independent, so the order changes")
-    c("  // no bit, and all lanes of a warp read the same word.  Returns the WRMS")
-    c("  // error norm and leaves the increment sum_j M_j K_j in S[DY..]; bit 1 of")
-    c("  // status is set on a zero pivot.")
+    c("  // one thread walks the stage programs (coop::attempt_prog) on its own")
+    c("  // cell; all lanes of a warp read the same word.  Returns the WRMS error")
+    c("  // norm and leaves the increment sum_j M_j K_j in S[DY..]; bit 1 of status")
+    c("  // is set on a zero pivot.")
     c("  template <class SA, class KA>")
     c("  __device__ __forceinline__ static double attempt(SA& S, const KA& k, double h, int& status) {")
     c("    for (int r = 0; r < NR; ++r) S[KT + r] = k(r);")
@@ -703,27 +690,7 @@ def _emit_table_attempt_head(c, coop, C):
     for (st, j), slot in coop["cterm_slot"].items():
         cv = C[(st - 1) * (st - 2) // 2 + j - 1]
         c(f"    S[{slot}] = {_lit(cv)} / h;    // c{st}{j} / h")
-    c("    bool ok = true;")
-    c("    const int steps = coop::stage_step[NSTAGE];")
-    c("    for (int s = 0; s < steps; ++s) {")
-    c("      const unsigned long long* __restrict__ row = coop::sched + (size_t)s * 32;")
-    c("      for (int j = 0; j < 32; ++j) {")
-    c("        const unsigned long long w = __ldg(row + j);")
-    c("        const unsigned lo = (unsigned)w, hi = (unsigned)(w >> 32);")
-    c("        const unsigned out = lo & 0xffffu;")
-    c("        if (out == 0xffffu) break;          // a step's idle lanes come last")
-    c("        if (hi >> 31) {")
-    c("          const double v = S[out];")
-    c("          ok = ok && (v != 0.0);")
-    c("          S[out] = 1.0 / v;")
-    c("        } else {")
-    c("          const double a = __longlong_as_double(__double_as_longlong(S[(lo >> 16) & 0x7fffu]) ^")
-    c("                                                ((long long)(lo >> 31) << 63));")
-    c("          S[out] = fma(a, S[hi & 0xffffu], S[(hi >> 16) & 0x7fffu]);")
-    c("        }")
-    c("      }")
-    c("    }")
-    c("    if (!ok) status |= 1;")
+    c("    if (!mkpp::run_program(S, coop::attempt_prog, coop::ATTEMPT_OPS)) status |= 1;")
 
 
 def _emit_coop(c, plan, coop, nv, ns, stages, C, M, E, K0, Y, FS, DY):
@@ -750,10 +717,19 @@ def _emit_coop(c, plan, coop, nv, ns, stages, C, M, E, K0, Y, FS, DY):
     for st_ in sched:
         offs.append(offs[-1] + len(st_))
     t(f"static __device__ const int stage_step[{len(offs)}] = {{{', '.join(map(str, offs))}}};")
+    # Numerators of the slots from CB + 3 on that depend on the step size.
+    nums = ["1.0"] + [_lit(C[(st - 1) * (st - 2) // 2 + j - 1]) for st, j in cterm_slot]
+    assert list(cterm_slot.values()) == [CB + 4 + i for i in range(len(cterm_slot))]
+    t(f"constexpr int H_TERMS = {len(nums)};")
+    t(f"static __device__ const double h_num[{len(nums)}] = {{{', '.join(nums)}}};")
     words = []
     for ops, st_ in zip(progs, sched):
         words += warp_schedule.encode(ops, st_)
     _c_u64_array(t, "sched", words)
+    if coop["seq_ops"] is not None:
+        ops = coop["seq_ops"]
+        t(f"constexpr int ATTEMPT_OPS = {len(ops)};")
+        _c_u64_array(t, "attempt_prog", warp_schedule.encode(ops, [[i] for i in range(len(ops))], lanes=1))
     if coop["adj_ops"] is not None:
         ops = coop["adj_ops"]
         t(f"constexpr int ADJ_OPS = {len(ops)};")
@@ -772,74 +748,25 @@ def _emit_coop(c, plan, coop, nv, ns, stages, C, M, E, K0, Y, FS, DY):
     plan._coop_programs = (progs, sched, {"CB": CB, "nconst": nconst, "literals": dict(literals),
                                           "cterm_slot": dict(cterm_slot), "Y": Y, "K0": K0, "FS": FS,
                                           "DY": DY, "KT": Mech_KT, "C": list(C), "slots": CB + nconst})
-    c("  // Run steps [s_begin, s_end) of the static warp schedule on S: one")
-    c("  // uniform operation S[out] = fma(+-S[a], S[b], S[c]) (or a pivot")
-    c("  // reciprocal) per lane and step, a warp barrier between steps.  The words")
-    c("  // of the next SCHED_AHEAD steps are in flight while the current ones")
-    c("  // execute; words past the end read as idle lanes.  Returns false if a")
-    c("  // reciprocal met a zero pivot.")
-    c("  static constexpr int SCHED_AHEAD = 8;")
-    c("  __device__ __forceinline__ static bool run_schedule(double* S, int s_begin, int s_end, unsigned lane) {")
-    c("    const unsigned long long* __restrict__ T = coop::sched;")
-    c("    bool ok = true;")
-    c("    unsigned long long cur[SCHED_AHEAD];")
-    c("    #pragma unroll")
-    c("    for (int j = 0; j < SCHED_AHEAD; ++j) {")
-    c("      const int s = s_begin + j;")
-    c("      cur[j] = s < s_end ? __ldg(T + (size_t)s * 32 + lane) : 0xffffull;")
-    c("    }")
-    c("    for (int s0 = s_begin; s0 < s_end; s0 += SCHED_AHEAD) {")
-    c("      unsigned long long nxt[SCHED_AHEAD];")
-    c("      #pragma unroll")
-    c("      for (int j = 0; j < SCHED_AHEAD; ++j) {")
-    c("        const int s = s0 + SCHED_AHEAD + j;")
-    c("        nxt[j] = s < s_end ? __ldg(T + (size_t)s * 32 + lane) : 0xffffull;")
-    c("      }")
-    c("      #pragma unroll")
-    c("      for (int j = 0; j < SCHED_AHEAD; ++j) {")
-    c("        const unsigned long long w = cur[j];")
-    c("        const unsigned lo = (unsigned)w, hi = (unsigned)(w >> 32);")
-    c("        const unsigned out = lo & 0xffffu;")
-    c("        if (out != 0xffffu) {")
-    c("          if (hi >> 31) {")
-    c("            const double v = S[out];")
-    c("            ok = ok && (v != 0.0);")
-    c("            S[out] = 1.0 / v;")
-    c("          } else {")
-    c("            // Negation flips the sign bit: exact, like -x in the per-thread code.")
-    c("            const double a = __longlong_as_double(__double_as_longlong(S[(lo >> 16) & 0x7fffu]) ^")
-    c("                                                  ((long long)(lo >> 31) << 63));")
-    c("            S[out] = fma(a, S[hi & 0xffffu], S[(hi >> 16) & 0x7fffu]);")
-    c("          }")
-    c("        }")
-    c("        __syncwarp();")
-    c("      }")
-    c("      #pragma unroll")
-    c("      for (int j = 0; j < SCHED_AHEAD; ++j) cur[j] = nxt[j];")
-    c("    }")
-    c("    return ok;")
+    c("  // The constant slots of a cell's store, once before its first attempt.")
+    c("  __device__ __forceinline__ static void coop_constants(double* S, unsigned lane) {")
+    c("    for (int i = lane; i < NCONST; i += 32) S[CB + i] = coop::const_val[i];")
+    c("    __syncwarp();")
     c("  }")
     c("")
-    c("  // One attempt by a whole warp on the cell held in shared memory S")
-    c("  // (COOP_SLOTS doubles; the rate constants in the KT slots).  Same values")
-    c("  // as attempt(); the error norm is summed by lane 0 in species order.")
-    c("  // Returns err on every lane.")
-    c("  template <class KA>")
-    c("  __device__ __forceinline__ static double attempt_coop(double* S, const KA& k, double h, int& status,")
-    c("                                                       unsigned lane) {")
-    c("    (void)k;")
+    c("  // One attempt by a whole warp on the cell held in S (COOP_SLOTS doubles;")
+    c("  // the rate constants in the KT slots, coop_constants() done); run executes")
+    c("  // a warp program.  Same values")
+    c("  // as attempt(); every lane sums the error norm in species order.  Returns")
+    c("  // err on every lane.")
+    c("  template <class Run>")
+    c("  __device__ __forceinline__ static double attempt_coop(double* S, double h, int& status, unsigned lane,")
+    c("                                                       const Run& run) {")
     c("    namespace T = coop;")
-    c("    for (int i = lane; i < NCONST; i += 32) S[CB + i] = T::const_val[i];")
+    c("    // 1/(gamma h) and the c_ij/h, one division of the whole warp.")
+    c("    if (lane < T::H_TERMS) S[CB + 3 + lane] = T::h_num[lane] / (lane == 0 ? GAMMA * h : h);")
     c("    __syncwarp();")
-    c("    if (lane == 0) {")
-    c("      S[CB + 3] = 1.0 / (GAMMA * h);")
-    for (st, j), slot in cterm_slot.items():
-        cv = C[(st - 1) * (st - 2) // 2 + j - 1]
-        c(f"      S[{slot}] = {_lit(cv)} / h;    // c{st}{j} / h")
-    c("    }")
-    c("    __syncwarp();")
-    c("    bool ok = true;")
-    c("    for (int st = 0; st < NSTAGE; ++st) ok = run_schedule(S, T::stage_step[st], T::stage_step[st + 1], lane) && ok;")
+    c("    const bool ok = run(S, T::sched, T::stage_step[NSTAGE], lane);")
     c("    if (__any_sync(0xffffffffu, !ok)) status |= 1;")
     mterms = [(M[j], j) for j in range(stages) if M[j] != 0.0]
     eterms = [(E[j], j) for j in range(stages) if E[j] != 0.0]
@@ -867,13 +794,10 @@ def _emit_coop(c, plan, coop, nv, ns, stages, C, M, E, K0, Y, FS, DY):
     c(f"      S[Q + i] = ({lin(eterms)}) / sc;")
     c("    }")
     c("    __syncwarp();")
-    c("    double err = 0.0;")
-    c("    if (lane == 0) {")
-    c("      double err_sq = 0.0;")
-    c("      for (int i = 0; i < NV; ++i) err_sq = fma(S[Q + i], S[Q + i], err_sq);")
-    c(f"      err = fmax(sqrt(err_sq / {ns}.0), 1.0e-10);")
-    c("    }")
-    c("    return __shfl_sync(0xffffffffu, err, 0);")
+    c("    double err_sq = 0.0;")
+    c("    #pragma unroll 8")
+    c("    for (int i = 0; i < NV; ++i) err_sq = fma(S[Q + i], S[Q + i], err_sq);")
+    c(f"    return fmax(sqrt(err_sq / {ns}.0), 1.0e-10);")
     c("  }")
     for line in tlm_code.lines:
         c(line)
@@ -1154,10 +1078,13 @@ def emit_mechanism(plan: ReducedPlan, table: bool | None = None) -> str:
           + ", ".join(str(x) for x in plan.fixed_phys) + "}; return t[i]; }")
     else:
         c("  __host__ __device__ static constexpr int fix_phys(int) { return 0; }")
-    c(f"  __host__ __device__ static constexpr double atol_v(int i) {{ constexpr double t[{nv}] = {{"
-      + ", ".join(_lit(plan.atol[p]) for p in plan.var_phys) + "}; return t[i]; }")
-    c(f"  __host__ __device__ static constexpr double rtol_v(int i) {{ constexpr double t[{nv}] = {{"
-      + ", ".join(_lit(plan.rtol[p]) for p in plan.var_phys) + "}; return t[i]; }")
+    # (One tolerance for all species is a literal: the cooperative attempt
+    # indexes by lane, which would put a table on the stack.)
+    for tol in ("atol", "rtol"):
+        vals = [_lit(getattr(plan, tol)[p]) for p in plan.var_phys]
+        body = f"(void)i; return {vals[0]};" if len(set(vals)) == 1 else \
+            f"constexpr double t[{nv}] = {{{', '.join(vals)}}}; return t[i];"
+        c(f"  __host__ __device__ static constexpr double {tol}_v(int i) {{ {body} }}")
     # Tolerances of every species in physical order, the reference's
     # SolverKernels::atol[] / rtol[] (host queries; the solve uses the above).
     c(f"  static constexpr double ATOL[NS] = {{" + ", ".join(_lit(x) for x in plan.atol) + "};")

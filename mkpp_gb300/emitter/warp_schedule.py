@@ -27,14 +27,26 @@ is built with --fmad=false, so only its explicit fma() calls fuse), and a
 cell gives the same bits on either kernel.
 
 Dependencies are the read-after-write, write-after-read and write-after-write
-hazards on slots, in program order.  A list scheduler (longest remaining
-dependency path first) packs the operations into steps of at most 32; the
-device runs one step per warp barrier.  On SAPRC99 the LU alone keeps ~31
-lanes busy; the solves, whose row sums keep a fixed order, allow ~2.7.
+hazards on slots, in program order.  ``pipeline`` packs the operations into
+steps of at most 32 for the device loop of csrc/warp_engine.cuh, which stores a
+step's results during the next step and loads operands one step ahead: a value
+is readable from its slot two steps after the operation that makes it, and one
+step after it by the same lane alone, from the register that holds the lane's
+previous result ("forwarded").  SAPRC99's attempt takes 2288 steps, of which
+1722 are the dependence chain of its three solves, whose row sums keep a fixed
+order.
 
-Encoding, one 64-bit word per lane and step:
-  bits 0-15 out | 16-30 a | 31 negate a | 32-47 b | 48-62 c | 63 reciprocal.
-An idle lane holds out = 0xffff.
+``schedule`` is plain list scheduling for a machine whose step sees all
+earlier steps; the tests use it as the reference for the dependencies.
+
+Encoding, one 64-bit word per lane and step, four fields of a 14-bit slot and
+two flags below it, so that a field is a byte offset after one shift:
+  bits 0-15   a: slot * 4 + (negate the product)
+  bits 16-31  b: slot * 4 + (the lane's previous result instead)
+  bits 32-47  c: slot * 4 + (the lane's previous result instead)
+  bits 48-63  out: slot * 4 + 2 * (reciprocal of b) + (store nothing)
+Storing nothing is an idle lane, or a result that only the lane's next
+operation reads.
 """
 
 from __future__ import annotations
@@ -43,7 +55,9 @@ import heapq
 
 FMA, RCP = 1, 2
 LANES = 32
-IDLE = 0xFFFF
+AHEAD = 8             # steps per unrolled group of the device loop
+IDLE = 1 << 48        # word of an idle lane
+PREV = -1             # operand: the lane's previous result
 
 
 class Program:
@@ -189,23 +203,167 @@ def schedule(ops, lanes: int = LANES) -> list[list[int]]:
     return steps
 
 
+LOAD = 2              # steps from an operation to a reader through its slot
+
+
+def pipeline(ops, lanes: int = LANES) -> list[list[int | None]]:
+    """Steps of `lanes` entries (an operation or None) for the device loop.
+    Priority: longest remaining path, a sum's next term one step after, any
+    other reader LOAD steps."""
+    n = len(ops)
+    raw: list[list[int]] = []
+    raw_succ: list[list[int]] = [[] for _ in range(n)]
+    other_succ: list[list[tuple[int, int]]] = [[] for _ in range(n)]
+    left = [0] * n
+    last: dict = {}
+    readers: dict = {}
+    for i, op in enumerate(ops):
+        reads, (out,) = _locations(op)
+        r = sorted({last[x] for x in reads if x in last})
+        raw.append(r)
+        # A slot's next writer may share the step of its readers (they have
+        # loaded it before), and follows an earlier writer.
+        after = {q: 0 for q in readers.get(out, ()) if q not in r}
+        if out in last and last[out] not in r:
+            after[last[out]] = 1
+        for j in r:
+            raw_succ[j].append(i)
+        for j, lag in after.items():
+            other_succ[j].append((i, lag))
+        left[i] = len(r) + len(after)
+        for x in reads:
+            readers.setdefault(x, []).append(i)
+        last[out], readers[out] = i, []
+    tail = [1] * n
+    for i in range(n - 1, -1, -1):
+        for t in raw_succ[i]:
+            lag = 1 if ops[t][0] == RCP or ops[t][4] == ops[i][1] else LOAD
+            tail[i] = max(tail[i], lag + tail[t])
+        for t, lag in other_succ[i]:
+            tail[i] = max(tail[i], lag + tail[t])
+    step, lane, earliest = [-1] * n, [-1] * n, [0] * n
+    from_slots = {0: [i for i in range(n) if left[i] == 0]}   # step -> operations ready then
+    forwarded: dict[int, list[tuple[int, int]]] = {}          # step -> (operation, the one it follows)
+    ready: list[tuple[int, int]] = []
+    s = done = 0
+
+    def release(i):
+        at = max([earliest[i]] + [step[j] + LOAD for j in raw[i]])
+        if raw[i]:
+            j = max(raw[i], key=lambda q: step[q])
+            f = step[j] + 1
+            square = ops[i][0] == FMA and ops[i][2] == ops[i][3] == ops[j][1]   # one factor can be forwarded
+            if (s < f < at and f >= earliest[i] and not square
+                    and all(step[q] + LOAD <= f for q in raw[i] if q != j)):
+                forwarded.setdefault(f, []).append((i, j))
+        if at <= s:
+            heapq.heappush(ready, (-tail[i], i))
+        else:
+            from_slots.setdefault(at, []).append(i)
+
+    def place(i):
+        step[i] = s
+        for t in raw_succ[i]:
+            left[t] -= 1
+            if left[t] == 0:
+                release(t)
+        for t, lag in other_succ[i]:
+            earliest[t] = max(earliest[t], s + lag)
+            left[t] -= 1
+            if left[t] == 0:
+                release(t)
+
+    while done < n:
+        for i in from_slots.pop(s, ()):
+            if step[i] < 0:
+                heapq.heappush(ready, (-tail[i], i))
+        follow = sorted((-tail[i], i, j) for i, j in forwarded.pop(s, ()))
+        used: set[int] = set()
+        anywhere = []
+        f = count = 0
+        while count < lanes and (ready or f < len(follow)):
+            if f < len(follow) and (not ready or follow[f][:2] <= ready[0]):
+                _, i, j = follow[f]
+                f += 1
+                if lane[j] in used:
+                    continue
+                lane[i] = lane[j]
+                used.add(lane[i])
+            else:
+                i = heapq.heappop(ready)[1]
+                if step[i] >= 0:
+                    continue
+                anywhere.append(i)
+            place(i)
+            count += 1
+        rest = (q for q in range(lanes) if q not in used)
+        for i in anywhere:
+            lane[i] = next(rest)
+        done += count
+        s += 1
+    rows: list[list[int | None]] = [[None] * lanes for _ in range(s)]
+    for i in range(n):
+        rows[step[i]][lane[i]] = i
+    return rows
+
+
 def encode(ops, steps, lanes: int = LANES) -> list[int]:
-    """steps x lanes words, idle lanes marked."""
-    words = []
-    for batch in steps:
-        row = [IDLE] * lanes
-        for lane, i in enumerate(batch):
-            kind, out, a, b, c, neg = ops[i]
-            assert 0 <= out < IDLE and 0 <= a < 32768 and 0 <= b < 65536 and 0 <= c < 32768
-            row[lane] = out | (a << 16) | (neg << 31) | (b << 32) | (c << 48) | ((kind == RCP) << 63)
-        words += row
-    return words
+    """steps x lanes words (a step lists the operations of its lanes, None or
+    missing for an idle lane).  An operand whose writer is the lane's
+    previous operation, one step before, is taken from the lane's register,
+    and a result that nothing else reads is not stored.  With several lanes
+    an odd number of steps is filled up with an idle one, and two steps'
+    words of a lane are side by side."""
+    where = {}
+    for s, row in enumerate(steps):
+        for q, i in enumerate(row):
+            if i is not None:
+                where[i] = (s, q)
+    fields: list = [None] * len(ops)
+    stored = [False] * len(ops)
+    last: dict = {}
+    for i, (kind, out, a, b, c, neg) in enumerate(ops):
+        if kind == RCP:
+            a, b, c = 0, b or out, 0
+        reads = [b] if kind == RCP else [a, b, c]
+        prev = {x for x in reads if x in last and where[last[x]] == (where[i][0] - 1, where[i][1])}
+        assert len(prev) <= 1
+        if kind == FMA and a in prev and a != b:
+            a, b = b, a
+        x_b = b in prev and not (kind == FMA and a == b)
+        x_c = kind == FMA and c in prev
+        from_slot = ([a] if kind == FMA else []) + ([] if x_b else [b]) + ([c] if kind == FMA and not x_c else [])
+        for x in from_slot:
+            if x in last:
+                assert lanes == 1 or where[last[x]][0] <= where[i][0] - LOAD
+                stored[last[x]] = True
+        fields[i] = (a, PREV if x_b else b, PREV if x_c else c)
+        last[out] = i
+    for i in last.values():
+        stored[i] = True
+    rows = []
+    for row in list(steps) + [[]] * (len(steps) % 2 if lanes > 1 else 0):
+        line = [IDLE] * lanes
+        for q, i in enumerate(row):
+            if i is None:
+                continue
+            kind, out, _, _, _, neg = ops[i]
+            a, b, c = fields[i]
+            assert all(PREV <= x < 1 << 14 for x in (out, a, b, c)) and a >= 0
+            lo = (a << 2 | bool(neg)) | (max(b, 0) << 2 | (b == PREV)) << 16
+            hi = (max(c, 0) << 2 | (c == PREV)) | (out << 2 | (kind == RCP) << 1 | (not stored[i])) << 16
+            line[q] = lo | hi << 32
+        rows.append(line)
+    if lanes == 1:
+        return [line[0] for line in rows]
+    return [line[q] for s in range(0, len(rows), 2) for q in range(lanes) for line in rows[s:s + 2]]
 
 
 def decode(word: int) -> tuple[int, int, int, int, int, int]:
-    """(kind, out, a, b, c, neg) of one word; kind 0 for an idle lane."""
-    out = word & 0xFFFF
-    if out == IDLE:
-        return 0, out, 0, 0, 0, 0
-    kind = RCP if word >> 63 else FMA
-    return kind, out, (word >> 16) & 0x7FFF, (word >> 32) & 0xFFFF, (word >> 48) & 0x7FFF, (word >> 31) & 1
+    """(kind, out, a, b, c, neg) of one word; kind 0 for a lane that stores
+    nothing, operand -1 for the lane's previous result."""
+    a, b, c, out = ((word >> 16 * f) & 0xFFFF for f in range(4))
+    if out & 1:
+        return 0, out >> 2, 0, 0, 0, 0
+    b_, c_ = (PREV if x & 1 else x >> 2 for x in (b, c))
+    return RCP if out & 2 else FMA, out >> 2, a >> 2, b_, c_, a & 1
