@@ -49,30 +49,14 @@ def lib_path(mech: str) -> Path:
 # the unrolled attempt of a large mechanism takes one to two minutes of
 # cicc + ptxas per kernel.  The heaviest units come first.
 UNITS = ("mkpp_adjoint.cu", "mkpp_checkpoint.cu", "mkpp_replay.cu", "mkpp_tangent.cu", "mkpp_capi.cu",
-         "mkpp_plain.cu", "mkpp_persist4.cu", "mkpp_tail.cu", "mkpp_eval.cu", "mkpp_coop.cu", "mkpp_diff.cu")
-
-
-# Units of a table-driven mechanism (too large to unroll, such as TS1): its
-# unrolled F/J evaluation kernels would take minutes to compile, so its
-# evaluation entries walk a table instead (mkpp_eval_table.cu).
-UNROLLED_ONLY = ("mkpp_eval.cu",)
-
-
-def is_table(mech: str) -> bool:
-    """True if the mechanism's generated header walks tables instead of
-    unrolled code (read from the header, which the emitter writes first)."""
-    return "TABLE_ATTEMPT = true" in (GEN / f"{mech}.cuh").read_text()
-
-
-def units(mech: str) -> tuple[str, ...]:
-    if is_table(mech):
-        return tuple(u for u in UNITS if u not in UNROLLED_ONLY) + ("mkpp_eval_table.cu",)
-    return UNITS
+         "mkpp_plain.cu", "mkpp_persist4.cu", "mkpp_tail.cu", "mkpp_eval.cu", "mkpp_coop.cu", "mkpp_coop_sweeps.cu",
+         "mkpp_diff.cu")
 
 
 def _sources(mech: str) -> list[Path]:
-    return [*(CSRC / u for u in units(mech)), CSRC / "capi_common.cuh", CSRC / "solver.cuh", CSRC / "eval_common.cuh",
-            CSRC / "mkpp_device.cuh", CSRC / "warp_engine.cuh", GEN / f"{mech}.cuh", INCLUDE / "mkpp.h", Path(__file__)]
+    return [*(CSRC / u for u in UNITS), CSRC / "capi_common.cuh", CSRC / "solver.cuh",
+            CSRC / "mkpp_device.cuh", CSRC / "warp_engine.cuh", CSRC / "coop_sweeps.cuh", GEN / f"{mech}.cuh", INCLUDE / "mkpp.h",
+            Path(__file__)]
 
 
 def _stale(mech: str) -> bool:
@@ -125,7 +109,7 @@ def _link(mech: str, objs: list[Path]) -> Path:
 def compile_mechanism(mech: str, verbose: bool = False, extra: list[str] | None = None) -> Path:
     """Compile the units of one mechanism in parallel and link the library."""
     LIB.mkdir(parents=True, exist_ok=True)
-    us = units(mech)
+    us = UNITS
     with ThreadPoolExecutor(max_workers=len(us)) as ex:
         objs = list(ex.map(lambda u: _compile_unit(mech, u, verbose), us))
     return _link(mech, objs)

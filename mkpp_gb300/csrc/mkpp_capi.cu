@@ -147,8 +147,12 @@ struct Tuning {
   // lanes' 6.2 M in four host steps of 65536.  A table-driven mechanism (TS1)
   // is always faster there: 79 against 293 ms for 4096 cells.  A mechanism
   // with few operations per attempt spends them on the parts that every lane
-  // of the warp repeats, so it stays on lanes.
-  int coop_cells = Mech::TABLE_ATTEMPT ? INT32_MAX : Mech::LU_FMA > 2000 ? 40000 : 0;
+  // of the warp repeats: saprc99_mini wins up to 8192 cells (2500 cells: 1.38
+  // against 3.14 ms; 32768: 8.8 against 7.2 ms), one whose lanes keep their
+  // store in registers a few hundred (small_strato: 72 cells 1.8 against 3.1
+  // ms, 4096 cells 6.1 against 3.5; Chapman: 0.50 against 0.60 ms, 2.1 against
+  // 0.67).
+  int coop_cells = Mech::TABLE_ATTEMPT ? INT32_MAX : Mech::LU_FMA > 2000 ? 40000 : StoreInfo::kTile ? 10000 : 600;
 };
 
 Tuning& tuning() {
@@ -179,7 +183,7 @@ int resident_blocks() {
   return std::max(1, per_sm);
 }
 
-constexpr size_t kCoopSmem = (size_t)Mech::COOP_SLOTS * sizeof(double);
+constexpr size_t kCoopSmem = (size_t)Mech::WARP_SLOTS * sizeof(double);
 
 LaunchConfig g_config;
 
@@ -227,7 +231,8 @@ int launch_rates(size_t cells, const double* conc, const double* temp, const dou
   a.clw = clw;
   a.ktab = ktab;
   a.status = status;
-  mkpp::rate_constant_kernel<Mech><<<launch_grid(cells, 128), 128, 0, stream>>>(a);
+  if (status && cudaMemsetAsync(status, 0, cells * sizeof(int), stream) != cudaSuccess) return MKPP_ERROR_DEVICE;
+  mkpp::rate_constant_kernel<Mech><<<dim3(launch_grid(cells, 128), Mech::RATE_PARTS), 128, 0, stream>>>(a);
   return cudaGetLastError() == cudaSuccess ? MKPP_SUCCESS : MKPP_ERROR_DEVICE;
 }
 
@@ -336,6 +341,10 @@ int noalloc_scratch(double** out) {
 }
 
 }  // namespace
+
+namespace mkpp_tu {
+int coop_cells() { return tuning().coop_cells; }
+}  // namespace mkpp_tu
 
 extern "C" {
 

@@ -1,0 +1,56 @@
+// The differentiation kernels with a warp per cell, of one mechanism library.
+#include "capi_common.cuh"
+#include "coop_sweeps.cuh"
+
+namespace mkpp_tu {
+
+namespace {
+
+// Launches `kernel` with one warp per block, as many as the cells and the
+// shared memory of the SMs allow.
+template <class Kernel, class... Args>
+int launch_warps(Kernel kernel, size_t slots, int cells, unsigned* next, cudaStream_t stream, const Args&... args) {
+  const size_t smem = slots * sizeof(double);
+  int per_sm = 0;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 32, smem) != cudaSuccess || per_sm < 1)
+    return MKPP_ERROR_DEVICE;
+  if (cudaMemsetAsync(next, 0, sizeof(unsigned), stream) != cudaSuccess) return MKPP_ERROR_DEVICE;
+  kernel<<<std::min(cells, per_sm * sm_count()), 32, smem, stream>>>(args...);
+  return cudaGetLastError() == cudaSuccess ? MKPP_SUCCESS : MKPP_ERROR_DEVICE;
+}
+
+// A block's shared memory on sm_103.
+constexpr size_t kMaxSmem = 227 * 1024;
+constexpr size_t kSlots = std::max(std::max(Mech::WARP_SLOTS, Mech::ADJ_COOP_SLOTS), Mech::TLM_COOP_SLOTS);
+
+}  // namespace
+
+// Up to half the cells of a plain integrate: the sweeps' stores are larger, and
+// both forms spend about twice the operations per step.  small_strato's and
+// saprc99_mini's sweeps gain longer, as their lanes keep more slots than
+// registers hold: 2000 cells 7.3 against 9.8 ms (gradient) and 7.4 against 19
+// ms (tangent), 16384 cells 41 against 10 ms; saprc99_mini, 8192 cells 6.1
+// against 9.4 ms.
+bool sweep_on_warps(size_t cells) {
+  constexpr size_t kLeast = Mech::NLU > 20 ? (StoreInfo::kTile ? 10000 : 2000) : 0;
+  return kSlots * sizeof(double) <= kMaxSmem && coop_cells() > 0 &&
+         cells <= std::max((size_t)coop_cells() / 2, kLeast);
+}
+
+int launch_checkpoint_coop(mkpp::LaunchArgs a, const mkpp::CheckpointArgs& ck, unsigned* next, cudaStream_t stream) {
+  a.coop_next = next;
+  return launch_warps(mkpp::checkpoint_coop_kernel<Mech>, Mech::WARP_SLOTS, a.ncells, next, stream, a, ck);
+}
+
+int launch_adjoint_coop(const mkpp::AdjointArgs& a, const mkpp::CheckpointArgs& ck, unsigned* next,
+                        cudaStream_t stream) {
+  return launch_warps(mkpp::adjoint_coop_kernel<Mech>, Mech::ADJ_COOP_SLOTS, a.ncells, next, stream, a, ck, next);
+}
+
+int launch_tangent_coop(const mkpp::TangentArgs& a, const mkpp::CheckpointArgs& ck, unsigned* next,
+                        cudaStream_t stream) {
+  return launch_warps(mkpp::tangent_coop_kernel<Mech>, Mech::TLM_COOP_SLOTS, a.ncells, next, stream, a, ck, next);
+}
+
+}  // namespace mkpp_tu

@@ -32,11 +32,16 @@ struct CellRow {
   __device__ __forceinline__ double operator()(int s) const { return __ldg(base + (size_t)s * stride); }
 };
 
-// Writable strided row (used for the rate-constant table).
-struct CellRowOut {
+// Writable strided row of the rate-constant table, which notes whether every
+// value was finite.
+struct CheckedRowOut {
   double* __restrict__ base;
   size_t stride;
-  __device__ __forceinline__ void set(int r, double v) const { base[(size_t)r * stride] = v; }
+  bool ok;
+  __device__ __forceinline__ void set(int r, double v) {
+    base[(size_t)r * stride] = v;
+    ok = ok && isfinite(v);
+  }
 };
 
 // Rate constants read back from the (reactions x cells) table.

@@ -90,7 +90,7 @@ struct RateArgs {
   const double* rh;          // [ncells] or null (0.5)
   const double* clw;         // [ncells] or null (0.0)
   double* ktab;              // [NR][ncells]
-  int* status;               // [ncells] or null: non-finite inputs are flagged
+  int* status;               // [ncells] or null, zeroed: non-finite inputs are flagged
 };
 
 // ---------------------------------------------------------------------------
@@ -100,31 +100,34 @@ struct ZeroRow {
   __device__ __forceinline__ double operator()(int) const { return 0.0; }
 };
 
+// A thread has one cell and one part of the reactions (blockIdx.y), so that a
+// small call spreads over the SMs: FP64 transcendentals, whose instructions a
+// warp issues one per 64 cycles, bound it (SAPRC99, 100 cells: 263 us with all
+// 211 reactions on a thread).  With the parts the evaluation of 1001 TS1 cells
+// went from 0.94 to 0.32 ms, of 20000 SAPRC99 cells from 0.83 to 0.66 ms.
 template <class Mech>
-__global__ void __launch_bounds__(128, 1) rate_constant_kernel(RateArgs a) {
+__global__ void __launch_bounds__(128) rate_constant_kernel(RateArgs a) {
   const size_t n = (size_t)a.ncells;
-  for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < n; c += (size_t)gridDim.x * blockDim.x) {
-    const double T = a.temp ? a.temp[c] : Mech::ENV_T;
-    const double RHO = a.rho ? a.rho[c] : Mech::ENV_RHO;
-    const double RH = a.rh ? a.rh[c] : 0.5;
-    const double CLW = a.clw ? a.clw[c] : 0.0;
-    CellRow fix{a.conc + c, n};
-    CellRowOut k{a.ktab + c, n};
-    if (a.param) {
-      CellRow P{a.param + c, n};
-      Mech::rate_constants(P, fix, T, RHO, RH, CLW, k);
-    } else {
-      ZeroRow P;
-      Mech::rate_constants(P, fix, T, RHO, RH, CLW, k);
-    }
-    if (a.status) {
-      bool ok = finite(T) && finite(RHO);
-#pragma unroll 1
-      for (int s = 0; s < Mech::NS; ++s) ok = ok && finite(a.conc[c + n * s]);
-#pragma unroll 1
-      for (int r = 0; r < Mech::NR; ++r) ok = ok && finite(a.ktab[c + n * r]);
-      a.status[c] = ok ? CELL_SUCCESS : CELL_ERR_NON_FINITE_STATE;
-    }
+  const size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  if (c >= n) return;
+  const int part = blockIdx.y;
+  const double T = a.temp ? a.temp[c] : Mech::ENV_T;
+  const double RHO = a.rho ? a.rho[c] : Mech::ENV_RHO;
+  const double RH = a.rh ? a.rh[c] : 0.5;
+  const double CLW = a.clw ? a.clw[c] : 0.0;
+  CellRow fix{a.conc + c, n};
+  CheckedRowOut k{a.ktab + c, n, true};
+  if (a.param) {
+    CellRow P{a.param + c, n};
+    Mech::rate_constants_part(part, P, fix, T, RHO, RH, CLW, k);
+  } else {
+    ZeroRow P;
+    Mech::rate_constants_part(part, P, fix, T, RHO, RH, CLW, k);
+  }
+  if (a.status) {  // all CELL_SUCCESS before the launch
+    bool ok = k.ok && finite(T) && finite(RHO);
+    for (int s = part; s < Mech::NS; s += Mech::RATE_PARTS) ok = ok && finite(a.conc[c + n * s]);
+    if (!ok) a.status[c] = CELL_ERR_NON_FINITE_STATE;
   }
 }
 
@@ -485,6 +488,19 @@ __global__ void __launch_bounds__(kBlock, MINB) integrate_persistent_kernel(Laun
 // on either form.  A block is one warp, so that a few cells spread over the
 // SMs, and its cells come from a work counter.
 // ---------------------------------------------------------------------------
+// final_status() of a cell whose finite check the warp has shared.
+__device__ __forceinline__ int coop_status(bool fin, bool capped, bool zero_pivot) {
+  return !fin ? CELL_ERR_NUMERICAL_FAILURE
+              : (capped ? CELL_ERR_CONVERGENCE_FAILURE : (zero_pivot ? CELL_ERR_SINGULAR_MATRIX : CELL_SUCCESS));
+}
+
+// The warp's next number from a work counter, on every lane.
+__device__ __forceinline__ unsigned next_cell(unsigned* counter, unsigned lane) {
+  unsigned idx = 0;
+  if (lane == 0) idx = atomicAdd(counter, 1u);
+  return __shfl_sync(0xffffffffu, idx, 0);
+}
+
 // One cell on a whole warp, from the controller state ctl at host step
 // `step` (attempt and accept counts so far in nacc, nrej) to the end of its
 // last host step; the cell's state is in S[Y..] already.  Writes the state,
@@ -524,10 +540,7 @@ __device__ __forceinline__ void coop_integrate_cell(const LaunchArgs& a, double*
   for (int i = lane; i < Mech::NV; i += 32) a.conc[c + n * Mech::var_phys(i)] = S[Mech::Y + i];
   if (lane == 0) {
     if (a.dt_carry) a.dt_carry[c] = ctl.carry_out();
-    const int status = !fin ? CELL_ERR_NUMERICAL_FAILURE
-                            : (capped ? CELL_ERR_CONVERGENCE_FAILURE
-                                      : (zero_pivot ? CELL_ERR_SINGULAR_MATRIX : CELL_SUCCESS));
-    if (a.status) a.status[c] = status;
+    if (a.status) a.status[c] = coop_status(fin, capped, zero_pivot);
     if (a.n_accept) a.n_accept[c] = nacc;
     if (a.n_reject) a.n_reject[c] = nrej;
   }
@@ -545,9 +558,7 @@ __global__ void __launch_bounds__(32) integrate_coop_kernel(LaunchArgs a) {
   // Every pass takes a new counter value, so a warp makes at most count + 1
   // passes.
   for (unsigned pass = 0; pass <= count; ++pass) {
-    unsigned idx = 0;
-    if (lane == 0) idx = atomicAdd(a.coop_next, 1u);
-    idx = __shfl_sync(0xffffffffu, idx, 0);
+    const unsigned idx = next_cell(a.coop_next, lane);
     if (idx >= count) break;
     Controller ctl;
     size_t c;
@@ -601,7 +612,7 @@ __global__ void __launch_bounds__(32) integrate_coop_kernel(LaunchArgs a) {
 template <class Mech>
 __global__ void __launch_bounds__(kBlock, 2) integrate_split_kernel(LaunchArgs a, double* scratch) {
   constexpr int kWarps = kBlock / 32;
-  static_assert((size_t)kWarps * Mech::COOP_SLOTS <= StoreFor<Mech>::block_bytes / sizeof(double),
+  static_assert((size_t)kWarps * Mech::WARP_SLOTS <= StoreFor<Mech>::block_bytes / sizeof(double),
                 "the warps' stores fit in the block's scratch tile");
   unsigned smid;
   asm("mov.u32 %0, %%smid;" : "=r"(smid));  // the SM this block runs on
@@ -610,15 +621,13 @@ __global__ void __launch_bounds__(kBlock, 2) integrate_split_kernel(LaunchArgs a
     return;
   }
   const unsigned lane = threadIdx.x & 31u;
-  double* S = scratch + (size_t)blockIdx.x * Mech::NSLOTS * kBlock + (size_t)(threadIdx.x >> 5) * Mech::COOP_SLOTS;
+  double* S = scratch + (size_t)blockIdx.x * Mech::NSLOTS * kBlock + (size_t)(threadIdx.x >> 5) * Mech::WARP_SLOTS;
   const size_t n = (size_t)a.ncells;
   Mech::coop_constants(S, lane);
   // Every pass takes a new counter value, so a warp makes at most
   // split_cells + 1 passes.
   for (int pass = 0; pass <= a.split_cells; ++pass) {
-    unsigned idx = 0;
-    if (lane == 0) idx = atomicAdd(a.split_next, 1u);
-    idx = __shfl_sync(0xffffffffu, idx, 0);
+    const unsigned idx = next_cell(a.split_next, lane);
     if (idx >= (unsigned)a.split_cells) break;
     const long long cell = a.order[idx];
     if (cell < 0 || cell >= (long long)n) continue;  // an order entry out of range names no cell

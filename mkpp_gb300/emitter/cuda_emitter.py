@@ -89,6 +89,8 @@ def _sum_expr(init: str | None, terms: list[tuple[float, str]]) -> str:
 
 
 ILP_GROUP = 8
+# Reactions per block of the rate-constant kernel.
+RATE_PART = 8
 # Slot count above which the solver keeps a cell's working set in the global
 # tile rather than registers (kRegisterSlots in csrc/solver.cuh).
 REGISTER_SLOTS = 96
@@ -120,9 +122,11 @@ def _interleave(c, plan, ops, operands, scale):
 
 
 def _c_array(c, ctype, name, values):
-    vals = list(values) or [0]
-    body = ", ".join(str(v) for v in vals)
-    c(f"static __device__ const {ctype} {name}[{len(vals)}] = {{{body}}};")
+    vals = [str(v) for v in values] or ["0"]
+    c(f"static __device__ const {ctype} {name}[{len(vals)}] = {{")
+    for i in range(0, len(vals), 32):
+        c(f"    {', '.join(vals[i:i + 32])},")
+    c("};")
 
 
 def _c_u64_array(c, name, values):
@@ -132,6 +136,11 @@ def _c_u64_array(c, name, values):
     for r in rows:
         c(f"    {r},")
     c("};")
+
+
+def _shifted(ops, first, by):
+    """The operations with the slots from `first` on moved down."""
+    return [(op[0], *(x - by if x >= first else x for x in op[1:5]), op[5]) for op in ops]
 
 
 def _coop_build(plan, nv, stages, A, C, NewF, K0, Y, FS, DY, nslots, table=False, M=None):
@@ -149,17 +158,14 @@ def _coop_build(plan, nv, stages, A, C, NewF, K0, Y, FS, DY, nslots, table=False
     Q = nslots                      # rates q_r (then q_i of the error norm)
     D = nslots + nq                 # Jacobian partial derivatives
     CB = D + npart                  # constants: -0, +0, 1, 1/(gamma h), c_ij/h, literals
-    adj = None
+    # The table-driven adjoint's slots sit before the constants.  The
+    # cooperative kernel's store does without them: its slots from the
+    # constants on are `shift` lower.
+    adj = _adjoint_layout(CB, nv, nr, stages) if table else None
+    shift = 0
     if table:
-        # The table-driven adjoint's slots sit before the constants: lambda,
-        # the stage adjoints, the pending tendency adjoint, dL/dk, and
-        # temporaries (one per reaction, one per species, a few scalars).
-        adj = {"LAM": CB}
-        adj["KBAR"] = adj["LAM"] + nv
-        adj["FBAR"] = adj["KBAR"] + stages * nv
-        adj["KB"] = adj["FBAR"] + nv
-        adj["TMP"] = adj["KB"] + nr
-        CB = adj["TMP"] + nr + nv + 8
+        shift = adj["end"] - CB
+        CB = adj["end"]
     ZN, ZP, ONE, IG = CB, CB + 1, CB + 2, CB + 3
     cterm_slot = {}
     for st in range(2, stages + 1):
@@ -282,7 +288,8 @@ def _coop_build(plan, nv, stages, A, C, NewF, K0, Y, FS, DY, nslots, table=False
                     P.fma(kb + i, cterm_slot[(st, j)], K0 + (j - 1) * nv + i, kb + i)
         P.solve(plan, kb)
         progs.append(P.ops)
-    sched = [warp_schedule.pipeline(ops) for ops in progs]
+    warp = [_shifted(ops, CB, shift) for ops in progs]
+    sched = [warp_schedule.pipeline(ops) for ops in warp]
     # An idle step or two end each stage, so that the next one's first step
     # finds every result in its slot and steps pair up; the last stage fills
     # up the device loop's groups of steps.
@@ -301,17 +308,36 @@ def _coop_build(plan, nv, stages, A, C, NewF, K0, Y, FS, DY, nslots, table=False
         fun(P, Y)
         eval_ops = P.ops
         assert all(op[0] != warp_schedule.RCP for op in eval_ops)
-    nconst = 4 + len(cterm_slot) + len(literals)
     const_vals = ["-0.0", "0.0", "1.0", "0.0"] + ["0.0"] * len(cterm_slot) + [_lit(v) for v in literals]
+    nconst = len(const_vals)
     seq_ops = [op for ops in progs for op in ops] if table else None
-    return {"progs": progs, "sched": sched, "seq_ops": seq_ops, "npart": npart, "nq": nq, "Q": Q, "D": D, "CB": CB,
-            "nconst": nconst, "const_vals": const_vals, "literals": literals, "cterm_slot": cterm_slot,
+    return {"progs": progs, "warp": warp, "shift": shift, "sched": sched, "seq_ops": seq_ops,
+            "npart": npart, "nq": nq, "Q": Q, "D": D, "CB": CB, "nconst": nconst, "const_vals": const_vals, "literals": literals, "cterm_slot": cterm_slot,
             "KT": Mech_KT, "total": CB + nconst, "adj": adj, "adj_ops": adj_ops, "eval_ops": eval_ops,
             "A": A, "NewF": NewF}
 
 
+# Sets of temporaries that a warp's sweep programs take in turn: with one set,
+# every reaction would wait for the one before it.
+SWEEP_SETS = 48
+
+
+def _adjoint_layout(base, nv, nr, stages, sets=1):
+    """Slots of the adjoint programs from `base` on: lambda, the stage
+    adjoints, the pending tendency adjoint, dL/dk, and temporaries (one per
+    reaction, one per species, `sets` sets of scalars, twice as many
+    products)."""
+    adj = {"LAM": base, "sets": sets}
+    adj["KBAR"] = adj["LAM"] + nv
+    adj["FBAR"] = adj["KBAR"] + stages * nv
+    adj["KB"] = adj["FBAR"] + nv
+    adj["TMP"] = adj["KB"] + nr
+    adj["end"] = adj["TMP"] + nr + nv + 6 * sets + 2 * sets
+    return adj
+
+
 def _adjoint_program(plan, P, nv, stages, A, C, M, NewF, K0, Y, KT, adj, cterm_slot):
-    """The reverse of one accepted step as a sequential program: operation
+    """The reverse of one accepted step as a program: operation
     for operation the arithmetic of the unrolled ``adjoint_step``
     (``_emit_adjoint``), the same sums in the same order.  A term is a
     product of factors evaluated left to right; a first term with a
@@ -321,7 +347,17 @@ def _adjoint_program(plan, P, nv, stages, A, C, M, NewF, K0, Y, KT, adj, cterm_s
     nr = len(plan.reactions)
     LAM, KBAR, FBAR, KB, TMP = adj["LAM"], adj["KBAR"], adj["FBAR"], adj["KB"], adj["TMP"]
     TS, TY = TMP, TMP + nr                       # per-reaction s, per-species stage state
-    T_S, T_G, T_KS, T_H, T_M, T_T, T_X = (TMP + nr + nv + i for i in range(7))
+    sets = adj["sets"]
+    turn = [0, 0]
+
+    def scalars():
+        """Slots for s, g, k s, h, a monomial and x: the next set."""
+        turn[0] = (turn[0] + 1) % sets
+        return range(TMP + nr + nv + 6 * turn[0], TMP + nr + nv + 6 * turn[0] + 6)
+
+    def term_slot():
+        turn[1] = (turn[1] + 1) % (2 * sets)
+        return TMP + nr + nv + 6 * sets + turn[1]
 
     def product(dest, factors):
         """dest = f1 * f2 * ... left to right (one factor: a copy)."""
@@ -332,14 +368,14 @@ def _adjoint_program(plan, P, nv, stages, A, C, M, NewF, K0, Y, KT, adj, cterm_s
         for f in factors[2:]:
             P.mul(dest, dest, f)
 
-    def mono(expo, ybase):
-        """Slot of prod y^e: the product is formed in T_M if it has more than
-        one factor.  Called just before the term that uses it."""
+    def mono(expo, ybase, slot):
+        """Slot of prod y^e: the product is formed in `slot` if it has more
+        than one factor.  Called just before the term that uses it."""
         fac = [ybase(q) for q in sorted(expo) for _ in range(expo[q])]
         if len(fac) == 1:
             return fac[0]
-        product(T_M, fac)
-        return T_M
+        product(slot, fac)
+        return slot
 
     def accumulate(dest, terms):
         """dest = sum over (coef, make) of coef * product(make()): first term
@@ -350,24 +386,26 @@ def _adjoint_program(plan, P, nv, stages, A, C, M, NewF, K0, Y, KT, adj, cterm_s
                 if coef == 1.0:
                     product(dest, factors)
                 elif coef == -1.0:
-                    product(T_T, factors)
-                    P.fma(dest, T_T, P.one, P.zn, neg=True)
+                    t = term_slot()
+                    product(t, factors)
+                    P.fma(dest, t, P.one, P.zn, neg=True)
                 else:
                     product(dest, [P.lit(coef)] + factors)
             else:
-                product(T_T, factors)
+                t = term_slot()
+                product(t, factors)
                 if coef == 1.0:
-                    P.fma(dest, T_T, P.one, dest)
+                    P.fma(dest, t, P.one, dest)
                 elif coef == -1.0:
-                    P.fma(dest, T_T, P.one, dest, neg=True)
+                    P.fma(dest, t, P.one, dest, neg=True)
                 else:
-                    P.fma(dest, P.lit(coef), T_T, dest)
+                    P.fma(dest, P.lit(coef), t, dest)
 
     def dot(net, base):
         return [(float(co), (lambda i=i: [base + i])) for i, co in net]
 
-    def ymono_v(e2, vslot):
-        return lambda: ([mono(e2, lambda q: Y + q), vslot] if e2 else [vslot])
+    def ymono_v(e2, vslot, t_m):
+        return lambda: ([mono(e2, lambda q: Y + q, t_m), vslot] if e2 else [vslot])
 
     rx = [(r.index, _monomial_terms(r.reactants, v2l), [(v2l[s_], co) for s_, co in r.net]) for r in plan.reactions]
     ucol = [[] for _ in range(nv)]
@@ -393,11 +431,12 @@ def _adjoint_program(plan, P, nv, stages, A, C, M, NewF, K0, Y, KT, adj, cterm_s
         for ri, expo, net in rx:
             if not net or not expo:
                 continue
+            T_S, T_G, T_KS, T_H, T_M, _ = scalars()
             accumulate(T_S, dot(net, ub))
             gterms = []
             for j in sorted(expo):
                 coef, e2 = _dmono(expo, j)
-                gterms.append((coef, ymono_v(e2, vb + j)))
+                gterms.append((coef, ymono_v(e2, vb + j, T_M)))
             accumulate(T_G, gterms)
             P.fma(KB + ri, T_S, T_G, KB + ri)
             P.mul(T_KS, KT + ri, T_S)
@@ -406,7 +445,7 @@ def _adjoint_program(plan, P, nv, stages, A, C, M, NewF, K0, Y, KT, adj, cterm_s
                 hterms = []
                 for q in sorted(e1):
                     c2, e2 = _dmono(e1, q)
-                    hterms.append((c1 * c2, ymono_v(e2, vb + q)))
+                    hterms.append((c1 * c2, ymono_v(e2, vb + q, T_M)))
                 if hterms:
                     accumulate(T_H, hterms)
                     P.fma(LAM + p_, T_KS, T_H, LAM + p_)
@@ -419,7 +458,7 @@ def _adjoint_program(plan, P, nv, stages, A, C, M, NewF, K0, Y, KT, adj, cterm_s
                 continue
             accumulate(TS + ri, dot(net, FBAR))
             if expo:
-                P.fma(KB + ri, TS + ri, mono(expo, yslot), KB + ri)
+                P.fma(KB + ri, TS + ri, mono(expo, yslot, scalars()[4]), KB + ri)
             else:
                 P.fma(KB + ri, TS + ri, P.one, KB + ri)
         yb_terms = {j: [] for j in range(nv)}
@@ -432,6 +471,7 @@ def _adjoint_program(plan, P, nv, stages, A, C, M, NewF, K0, Y, KT, adj, cterm_s
                 yb_terms[j].append((coef, (lambda fac=fac: fac)))
         for j in range(nv):
             if yb_terms[j]:
+                T_X = scalars()[5]
                 accumulate(T_X, yb_terms[j])
                 P.fma(LAM + j, T_X, P.one, LAM + j)
                 for a, jj in aterms:
@@ -468,8 +508,9 @@ def _adjoint_program(plan, P, nv, stages, A, C, M, NewF, K0, Y, KT, adj, cterm_s
                         if a == 1.0:
                             P.fma(TY + q, kk, P.one, acc)
                         else:
-                            P.mul(T_T, kk, P.lit(a))
-                            P.fma(TY + q, T_T, P.one, acc)
+                            t = term_slot()
+                            P.mul(t, kk, P.lit(a))
+                            P.fma(TY + q, t, P.one, acc)
                         acc = TY + q
                 fterm(lambda q: TY + q, aterms)
             else:
@@ -478,7 +519,7 @@ def _adjoint_program(plan, P, nv, stages, A, C, M, NewF, K0, Y, KT, adj, cterm_s
                 P.zero(FBAR + j)
 
 
-def _tlm_build(plan, nv, stages, A, C, M, NewF, K0, Y, KT, base):
+def _tlm_build(plan, nv, stages, A, C, M, NewF, K0, Y, KT, base, sets=1):
     """Tangent of one accepted step of size h (forward mode), as a sequential
     program of uniform operations with its own slots and constants from
     `base` on.  With W = I/(gamma h) - J(y) and F_i = f(Y_i):
@@ -498,10 +539,20 @@ def _tlm_build(plan, nv, stages, A, C, M, NewF, K0, Y, KT, base):
     L["TY"] = L["DF"] + nv
     L["TD"] = L["TY"] + nv
     TT = L["TD"] + nv
-    TCB = TT + 8
+    TCB = TT + (8 if sets == 1 else 4 * sets)
     L["TCB"] = TCB
     DYT, DKR, DK, DF, TY, TD = L["DYT"], L["DKR"], L["DK"], L["DF"], L["TY"], L["TD"]
-    T_A, T_B, T_P = TT, TT + 1, TT + 2
+    turn = [0, 0]
+
+    def pair():
+        """Two scalars of the next set."""
+        turn[0] = (turn[0] + 1) % sets
+        return TT + 2 * turn[0], TT + 2 * turn[0] + 1
+
+    def term_slot():
+        turn[1] = (turn[1] + 1) % (2 * sets)
+        return TT + 2 * sets + turn[1]
+
     cterm = {}
     for st in range(2, stages + 1):
         for j in range(1, st):
@@ -544,8 +595,9 @@ def _tlm_build(plan, nv, stages, A, C, M, NewF, K0, Y, KT, base):
         P.zero(dest)
         for j in sorted(expo):
             c1, e2 = _dmono(expo, j)
-            product(T_P, ys_of(e2, yslot) + [vslot(j)])
-            add_scaled(dest, c1, T_P)
+            t = term_slot()
+            product(t, ys_of(e2, yslot) + [vslot(j)])
+            add_scaled(dest, c1, t)
 
     def hess(dest, expo, yslot, uslot, vslot):
         """dest = sum_p sum_q u_p d2m/dy_p dy_q (y) v_q"""
@@ -554,8 +606,9 @@ def _tlm_build(plan, nv, stages, A, C, M, NewF, K0, Y, KT, base):
             c1, e1 = _dmono(expo, p_)
             for q in sorted(e1):
                 c2, e2 = _dmono(e1, q)
-                product(T_P, ys_of(e2, yslot) + [uslot(p_), vslot(q)])
-                add_scaled(dest, c1 * c2, T_P)
+                t = term_slot()
+                product(t, ys_of(e2, yslot) + [uslot(p_), vslot(q)])
+                add_scaled(dest, c1 * c2, t)
 
     rx = [(r.index, _monomial_terms(r.reactants, v2l), [(v2l[s_], co) for s_, co in r.net]) for r in plan.reactions]
     for i in range(stages):
@@ -577,6 +630,7 @@ def _tlm_build(plan, nv, stages, A, C, M, NewF, K0, Y, KT, base):
             for ri, expo, net in rx:
                 if not net:
                     continue
+                T_A, T_B = pair()
                 if expo:
                     grad_dot(T_A, expo, ys, ds)
                     P.mul(T_A, KT + ri, T_A)
@@ -594,6 +648,7 @@ def _tlm_build(plan, nv, stages, A, C, M, NewF, K0, Y, KT, base):
         for ri, expo, net in rx:
             if not net or not expo:
                 continue
+            T_A, T_B = pair()
             grad_dot(T_A, expo, lambda q: Y + q, lambda q, i=i: K0 + i * nv + q)
             P.mul(T_A, DKR + ri, T_A)
             hess(T_B, expo, lambda q: Y + q, lambda p_, i=i: K0 + i * nv + p_, lambda q: DYT + q)
@@ -607,8 +662,79 @@ def _tlm_build(plan, nv, stages, A, C, M, NewF, K0, Y, KT, base):
                 add_scaled(DYT + q, M[i], DK + i * nv + q)
     nconst = 3 + len(cterm) + len(literals)
     const_vals = ["-0.0", "0.0", "1.0"] + ["0.0"] * len(cterm) + [_lit(v) for v in literals]
-    return {"ops": P.ops, "L": L, "cterm": cterm, "nconst": nconst, "const_vals": const_vals,
-            "total": TCB + nconst}
+    return {"ops": P.ops, "L": L, "cterm": cterm, "literals": literals, "nconst": nconst,
+            "const_vals": const_vals, "total": TCB + nconst}
+
+
+def _warp_sweeps(plan, nv, stages, C, M, K0, Y, coop):
+    """The adjoint and the tangent of one accepted step as warp programs on
+    the cooperative store, from the LU and the K_i that the attempt's
+    programs leave: the sequential programs' operations, with more
+    temporaries.  Slots follow the cooperative kernel's; literals that the
+    attempt does not have come last."""
+    total = coop["CB"] + coop["nconst"]
+    A, NewF, KT, CB = coop["A"], coop["NewF"], coop["KT"], coop["CB"]
+    nr = len(plan.reactions)
+    out = {}
+    for name in ("adj", "tlm"):
+        if name == "adj":
+            L = _adjoint_layout(total, nv, nr, stages, SWEEP_SETS)
+            end = L["end"]
+        else:
+            tlm = _tlm_build(plan, nv, stages, A, C, M, NewF, K0, Y, KT, total, SWEEP_SETS)
+            L, end = tlm["L"], tlm["L"]["TCB"]
+        extra: dict[float, int] = {}
+
+        def lit(v):
+            v = float(v)
+            return coop["literals"][v] if v in coop["literals"] else extra.setdefault(v, end + len(extra))
+
+        if name == "adj":
+            P = warp_schedule.Program(CB, CB + 1, CB + 2, lit)
+            _adjoint_program(plan, P, nv, stages, A, C, M, NewF, K0, Y, KT, L, coop["cterm_slot"])
+            ops = P.ops
+        else:
+            # The tangent's own constants are the attempt's.
+            same = {L["TCB"]: CB, L["TCB"] + 1: CB + 1, L["TCB"] + 2: CB + 2}
+            same.update({slot: coop["cterm_slot"][key] for key, slot in tlm["cterm"].items()})
+            same.update({slot: lit(v) for v, slot in tlm["literals"].items()})
+            ops = [(op[0], *(same.get(x, x) for x in op[1:5]), op[5]) for op in tlm["ops"]]
+        by = coop["shift"]
+        ops = _shifted(ops, CB, by)
+        L = {key: x - by if x >= CB else x for key, x in L.items()}
+        extra = {v: slot - by for v, slot in extra.items()}
+        end -= by
+        steps = warp_schedule.pipeline(ops)
+        steps += [[]]
+        steps += [[]] * (-len(steps) % warp_schedule.AHEAD)
+        out[name] = {"ops": ops, "steps": steps, "L": L, "end": end, "extra": extra, "slots": end + len(extra)}
+    return out
+
+
+def _emit_warp_sweeps(c, t, sweeps):
+    """Tables (into the coop namespace text t) and members of the warp forms
+    of adjoint_step and tlm_step."""
+    c("")
+    c("  // ---- adjoint and tangent of one accepted step on a warp ----")
+    c("  // Slots beyond WARP_SLOTS of the adjoint's and the tangent's stores.")
+    adj, tlm = sweeps["adj"], sweeps["tlm"]
+    for name, slot in (("W_LAM", adj["L"]["LAM"]), ("W_KB", adj["L"]["KB"]), ("W_DYT", tlm["L"]["DYT"]),
+                       ("W_DKR", tlm["L"]["DKR"]), ("ADJ_COOP_SLOTS", adj["slots"]), ("TLM_COOP_SLOTS", tlm["slots"])):
+        c(f"  static constexpr int {name} = {slot};")
+    for name, sw in sweeps.items():
+        t(f"constexpr int {name.upper()}_STEPS = {len(sw['steps'])};")
+        _c_u64_array(t, f"{name}_sched", warp_schedule.encode(sw["ops"], sw["steps"]))
+        _c_array(t, "double", f"{name}_lit", [_lit(v) for v in sw["extra"]])
+        step = {"adj": "adjoint", "tlm": "tangent"}[name]
+        c(f"  // adjoint_step() and tlm_step() after stages_coop() for the same step." if name == "adj" else "")
+        c(f"  __device__ __forceinline__ static void {step}_constants(double* S, unsigned lane) {{")
+        c(f"    for (int i = lane; i < {len(sw['extra'])}; i += 32) S[{sw['end']} + i] = coop::{name}_lit[i];")
+        c("    __syncwarp();")
+        c("  }")
+        c("  template <class Run>")
+        c(f"  __device__ __forceinline__ static void {step}_coop(double* S, unsigned lane, const Run& run) {{")
+        c(f"    run(S, coop::{name}_sched, coop::{name.upper()}_STEPS, lane);")
+        c("  }")
 
 
 def _emit_tlm(c, t, tlm, C):
@@ -709,6 +835,8 @@ def _emit_coop(c, plan, coop, nv, ns, stages, C, M, E, K0, Y, FS, DY):
     c(f"  static constexpr int CB = {CB};        // constants")
     c(f"  static constexpr int NCONST = {nconst};")
     c(f"  static constexpr int COOP_SLOTS = CB + NCONST;")
+    c(f"  static constexpr int WCB = {CB - coop['shift']};       // constants in the store of a warp")
+    c(f"  static constexpr int WARP_SLOTS = WCB + NCONST;")
     t = _Code()
     t("// Tables of the warp-cooperative attempt (device constant data).")
     t("namespace coop {")
@@ -723,7 +851,7 @@ def _emit_coop(c, plan, coop, nv, ns, stages, C, M, E, K0, Y, FS, DY):
     t(f"constexpr int H_TERMS = {len(nums)};")
     t(f"static __device__ const double h_num[{len(nums)}] = {{{', '.join(nums)}}};")
     words = []
-    for ops, st_ in zip(progs, sched):
+    for ops, st_ in zip(coop["warp"], sched):
         words += warp_schedule.encode(ops, st_)
     _c_u64_array(t, "sched", words)
     if coop["seq_ops"] is not None:
@@ -742,6 +870,9 @@ def _emit_coop(c, plan, coop, nv, ns, stages, C, M, E, K0, Y, FS, DY):
     tlm_code = _Code()
     _emit_tlm(tlm_code, t, tlm, C)
     plan._tlm = tlm
+    sweeps = _warp_sweeps(plan, nv, stages, C, M, K0, Y, coop)
+    plan._sweeps = sweeps
+    _emit_warp_sweeps(tlm_code, t, sweeps)
     t("}  // namespace coop")
     t("")
     plan._coop_tables = t.text()
@@ -750,24 +881,30 @@ def _emit_coop(c, plan, coop, nv, ns, stages, C, M, E, K0, Y, FS, DY):
                                           "DY": DY, "KT": Mech_KT, "C": list(C), "slots": CB + nconst})
     c("  // The constant slots of a cell's store, once before its first attempt.")
     c("  __device__ __forceinline__ static void coop_constants(double* S, unsigned lane) {")
-    c("    for (int i = lane; i < NCONST; i += 32) S[CB + i] = coop::const_val[i];")
+    c("    for (int i = lane; i < NCONST; i += 32) S[WCB + i] = coop::const_val[i];")
     c("    __syncwarp();")
     c("  }")
     c("")
-    c("  // One attempt by a whole warp on the cell held in S (COOP_SLOTS doubles;")
-    c("  // the rate constants in the KT slots, coop_constants() done); run executes")
-    c("  // a warp program.  Same values")
-    c("  // as attempt(); every lane sums the error norm in species order.  Returns")
-    c("  // err on every lane.")
+    c("  // The stages of an attempt by a whole warp on the cell held in S (the rate")
+    c("  // constants in the KT slots, coop_constants() done): the LU and the K_i of")
+    c("  // attempt(), bit for bit.  run executes a warp program.")
     c("  template <class Run>")
-    c("  __device__ __forceinline__ static double attempt_coop(double* S, double h, int& status, unsigned lane,")
-    c("                                                       const Run& run) {")
+    c("  __device__ __forceinline__ static void stages_coop(double* S, double h, int& status, unsigned lane,")
+    c("                                                    const Run& run) {")
     c("    namespace T = coop;")
     c("    // 1/(gamma h) and the c_ij/h, one division of the whole warp.")
-    c("    if (lane < T::H_TERMS) S[CB + 3 + lane] = T::h_num[lane] / (lane == 0 ? GAMMA * h : h);")
+    c("    if (lane < T::H_TERMS) S[WCB + 3 + lane] = T::h_num[lane] / (lane == 0 ? GAMMA * h : h);")
     c("    __syncwarp();")
     c("    const bool ok = run(S, T::sched, T::stage_step[NSTAGE], lane);")
     c("    if (__any_sync(0xffffffffu, !ok)) status |= 1;")
+    c("  }")
+    c("")
+    c("  // One attempt by a whole warp: same values as attempt(); every lane sums")
+    c("  // the error norm in species order.  Returns err on every lane.")
+    c("  template <class Run>")
+    c("  __device__ __forceinline__ static double attempt_coop(double* S, double h, int& status, unsigned lane,")
+    c("                                                       const Run& run) {")
+    c("    stages_coop(S, h, status, lane, run);")
     mterms = [(M[j], j) for j in range(stages) if M[j] != 0.0]
     eterms = [(E[j], j) for j in range(stages) if E[j] != 0.0]
 
@@ -801,6 +938,77 @@ def _emit_coop(c, plan, coop, nv, ns, stages, C, M, E, K0, Y, FS, DY):
     c("  }")
     for line in tlm_code.lines:
         c(line)
+
+
+def _eval_tables(plan) -> str:
+    """Tables of the evaluation kernels (csrc/mkpp_eval.cu), on physical
+    species: the rates q_r = k_r * y * ..., the tendencies as sums over
+    reactions, and per column of the dense Jacobian its partial derivatives
+    and, per row, the sum that makes the entry of -W (1/(gamma h) = 0).  The
+    factors and terms stand in the order of fun() and jac_w()."""
+    ns = plan.n_species
+    v2p = {i: p for i, p in enumerate(plan.var_phys)}
+    t = _Code()
+    t("// Tables of the evaluation kernels (device constant data).")
+    t("namespace eval {")
+    factors: list[int] = []
+
+    def product(codes):
+        """A product of k_r and these factors: where they start, how many."""
+        start = len(factors)
+        factors.extend(codes)
+        return start << 4 | len(codes)
+
+    rates = [product([s_ for s_, pw in r.reactants for _ in range(pw)]) for r in plan.reactions]
+    columns = {j: [] for j in range(ns)}     # column -> [(reaction, product)]
+    where = {}                               # (reaction, species) -> position in its column
+    for r in plan.reactions:
+        terms = list(r.reactants)
+        for x, (s_, pw) in enumerate(terms):
+            codes = []
+            for y, (s2, pw2) in enumerate(terms):
+                if x != y:
+                    codes += [s2] * pw2
+                elif pw2 > 1:
+                    codes += [0x8000 | pw2] + [s2] * (pw2 - 1)
+            where[(r.index, s_)] = len(columns[s_])
+            columns[s_].append((r.index, product(codes)))
+    f_rows = {i: [] for i in range(ns)}
+    entries = {(v2p[a], v2p[b]): [] for a, b in plan.w_slots}
+    for r in plan.reactions:
+        for s_, coef in r.net:
+            f_rows[s_].append((coef, r.index))
+            for s2, _pw in r.reactants:
+                entries[(s_, s2)].append((-coef, where[(r.index, s2)]))
+    f_ptr, f_term, f_coef = [0], [], []
+    for i in range(ns):
+        f_term += [q for _, q in f_rows[i]]
+        f_coef += [_lit(q) for q, _ in f_rows[i]]
+        f_ptr.append(len(f_term))
+    p_ptr, p_rate, p_product = [0], [], []
+    j_ptr, j_term, j_coef = [], [], []
+    for col in range(ns):
+        p_rate += [r for r, _ in columns[col]]
+        p_product += [q for _, q in columns[col]]
+        p_ptr.append(len(p_rate))
+        for row in range(ns):
+            terms = entries.get((row, col))
+            # 2: an entry of W, 1: on its diagonal
+            j_ptr.append(len(j_term) << 2 | (terms is not None) << 1 | (terms is not None and row == col))
+            j_term += [q for _, q in terms or []]
+            j_coef += [_lit(q) for q, _ in terms or []]
+    j_ptr.append(len(j_term) << 2)
+    t(f"constexpr int MAX_PARTIALS = {max(len(v) for v in columns.values())};   // of one column")
+    for name, ctype, vals in (("factor", "unsigned short", factors), ("rate", "unsigned", rates),
+                              ("f_ptr", "int", f_ptr), ("f_term", "unsigned short", f_term),
+                              ("f_coef", "double", f_coef), ("p_ptr", "int", p_ptr),
+                              ("p_rate", "unsigned short", p_rate), ("p_product", "unsigned", p_product),
+                              ("j_ptr", "unsigned", j_ptr), ("j_term", "unsigned short", j_term),
+                              ("j_coef", "double", j_coef)):
+        _c_array(t, ctype, name, vals)
+    t("}  // namespace eval")
+    t("")
+    return t.text()
 
 
 def _monomial_terms(reactants, v2l):
@@ -1106,13 +1314,26 @@ def emit_mechanism(plan: ReducedPlan, table: bool | None = None) -> str:
     c("  // Rate constants of every reaction (reaction index order).  P(n) is the")
     c("  // cell's runtime parameter n (photolysis J_n or external Rate slot n),")
     c("  // FIX(s) the concentration of fixed species s, T/RHO the cell's")
-    c("  // temperature and air density.")
+    c("  // temperature and air density.  In parts of a few reactions, which the")
+    c("  // rate kernel gives to different blocks.")
+    parts = [plan.reactions[i:i + RATE_PART] for i in range(0, nr, RATE_PART)]
+    c(f"  static constexpr int RATE_PARTS = {len(parts)};")
+    c("  template <class PA, class FA, class KO>")
+    c("  __device__ __forceinline__ static void rate_constants_part(int part, const PA& P, const FA& FIX, double T,")
+    c("                                                           double RHO, double RH, double CLW, KO& k) {")
+    c("    (void)T; (void)RHO; (void)RH; (void)CLW; (void)P; (void)FIX;")
+    c("    switch (part) {")
+    for i, part in enumerate(parts):
+        c(f"      case {i}:")
+        for r in part:
+            c(f"        k.set({r.index}, {_k_text(r.k)});")
+        c("        break;")
+    c("    }")
+    c("  }")
     c("  template <class PA, class FA, class KO>")
     c("  __device__ __forceinline__ static void rate_constants(const PA& P, const FA& FIX, double T, double RHO,")
     c("                                                      double RH, double CLW, KO& k) {")
-    c("    (void)T; (void)RHO; (void)RH; (void)CLW; (void)P; (void)FIX;")
-    for r in plan.reactions:
-        c(f"    k.set({r.index}, {_k_text(r.k)});")
+    c("    for (int p = 0; p < RATE_PARTS; ++p) rate_constants_part(p, P, FIX, T, RHO, RH, CLW, k);")
     c("  }")
     c("")
     # ---------------- storage layout
@@ -1209,6 +1430,12 @@ def emit_mechanism(plan: ReducedPlan, table: bool | None = None) -> str:
         c("    " + _accumulate(f"S[{slot}]", init, wterms[loc]))
     c("  }")
     c("")
+    if store_slots <= REGISTER_SLOTS:
+        slot_at = {plan.var_phys[a] + ns * plan.var_phys[b]: plan.lu_index[(a, b)] for a, b in plan.w_slots}
+        c("  // W slot of entry row + NS * column of the dense Jacobian, -1 for none.")
+        c(f"  __host__ __device__ static constexpr int w_slot(int e) {{ constexpr int t[{ns * ns}] = {{"
+          + ", ".join(str(slot_at.get(e, -1)) for e in range(ns * ns)) + "}; return t[e]; }")
+        c("")
     c("  // Physical (row, column) of every W slot, for the dense Jacobian.")
     c("  template <class Fn>")
     c("  __device__ __forceinline__ static void for_each_w_slot(Fn&& fn) {")
@@ -1407,7 +1634,7 @@ def emit_mechanism(plan: ReducedPlan, table: bool | None = None) -> str:
     c("")
     c(f"}}  // namespace mkpp_{name}")
     text = c.text()
-    return text.replace("struct Mech {", plan._coop_tables + "\nstruct Mech {", 1)
+    return text.replace("struct Mech {", plan._coop_tables + _eval_tables(plan) + "\nstruct Mech {", 1)
 
 
 def emit_host_header(plan) -> str:

@@ -1,8 +1,11 @@
-"""Calls that the cooperative kernel takes as a whole (GPU).
+"""Calls that the cooperative kernel takes as a whole, and the evaluation
+kernels, at the sizes where their splits end (GPU).
 
 A persistent call of few cells runs every cell on a whole warp; the plain form
 runs a thread per cell.  Both have to end bit-identical, with cells in a given
-order, cells flagged as not finite and the attempt cap reached included.
+order, cells flagged as not finite and the attempt cap reached included.  The
+evaluation kernels take 32 cells per block: their outputs of a cell do not
+depend on the number of cells around it.
 """
 
 import numpy as np
@@ -51,3 +54,21 @@ def test_cooperative_call_equals_plain(libs, mech, cells, dt, steps):
     assert (capped[0][1] != 0).any()
     for a, b in zip(*capped):
         assert np.array_equal(a, b, equal_nan=True)
+
+
+@pytest.mark.parametrize("mech", ["saprc99", "ts1"])
+def test_evaluation_does_not_depend_on_the_batch(libs, mech):
+    import torch
+
+    from mkpp_gb300.api import DeviceSolver
+
+    s = DeviceSolver(mech)
+    w = workloads.make(mech, 97, seed=6)
+    d = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()  # noqa: E731
+    conc = d(w.conc)
+    k, _ = s.rate_constants(conc, d(w.temp), d(w.rho), d(w.rh), None, d(w.param))
+    f, j = s.evaluate_rates(conc, k), s.evaluate_jacobian(conc, k)
+    for n in (1, 31, 32, 33, 64, 65):
+        sub, ks = conc[:, 97 - n:].contiguous(), k[:, 97 - n:].contiguous()
+        assert torch.equal(s.evaluate_rates(sub, ks), f[:, 97 - n:])
+        assert torch.equal(s.evaluate_jacobian(sub, ks), j[:, :, 97 - n:])

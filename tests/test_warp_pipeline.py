@@ -89,3 +89,60 @@ def test_device_loop_ends_as_program_order(mech):
             if lanes > 1:
                 assert np.array_equal(_device_loop(ws.encode(ops, steps, lanes), S, lanes), want)
         assert np.array_equal(_thread_loop(ws.encode(ops, [[i] for i in range(len(ops))], 1), S), want)
+
+
+@pytest.mark.parametrize("mech", ["chapman", "small_strato_rodas3", "saprc99_mini", "saprc99"])
+def test_warp_sweeps_equal_the_sequential_programs(mech):
+    """The warps' adjoint and tangent programs (more temporaries, the
+    attempt's constants) leave the results of the sequential ones, bit for
+    bit, in order and through the device loop."""
+    plan = load(mech)
+    cuda_emitter.emit_mechanism(plan)
+    _, _, info = plan._coop_programs
+    warp = plan._sweeps
+    tab = plan.tableau
+    nv, nr, stages = plan.n_var, len(plan.reactions), int(tab["stages"])
+    A, C, M, NewF = tab["A"], tab["C"], tab["M"], tab["NewF"]
+    K0, Y, KT, CB = info["K0"], info["Y"], info["KT"], info["CB"]
+    rng = np.random.default_rng(3)
+    base = max(w["slots"] for w in warp.values())   # the sequential layouts follow the warps' slots
+    size = 2 * base
+
+    # Sequential adjoint on its own layout, with the warp's literal slots.
+    literals = {**info["literals"], **warp["adj"]["extra"]}
+    adj = cuda_emitter._adjoint_layout(base, nv, nr, stages)
+    P = ws.Program(CB, CB + 1, CB + 2, lambda v: literals[float(v)])
+    cuda_emitter._adjoint_program(plan, P, nv, stages, A, C, M, NewF, K0, Y, KT, adj, info["cterm_slot"])
+    seq_t = cuda_emitter._tlm_build(plan, nv, stages, A, C, M, NewF, K0, Y, KT, base)
+
+    def store(extra):
+        S = np.zeros(size + base)
+        S[:info["slots"]] = np.random.default_rng(4).uniform(0.5, 1.5, info["slots"])
+        S[CB:CB + 3] = (-0.0, 0.0, 1.0)
+        for v, slot in {**info["literals"], **extra}.items():
+            S[slot] = v
+        return S
+
+    for name, ops, seq, ins, outs in (
+            ("adj", P.ops, adj, (("LAM", nv),), (("LAM", nv), ("KB", nr))),
+            ("tlm", seq_t["ops"], seq_t["L"], (("DYT", nv), ("DKR", nr)), (("DYT", nv),))):
+        w = warp[name]
+        given = {key: rng.uniform(-1.0, 1.0, n) for key, n in ins}
+        one, many = store(warp["adj"]["extra"] if name == "adj" else {}), store(w["extra"])
+        if name == "tlm":
+            t0 = seq_t["L"]["TCB"]
+            one[t0:t0 + 3] = (-0.0, 0.0, 1.0)
+            for key, slot in seq_t["cterm"].items():
+                one[slot] = one[info["cterm_slot"][key]]
+            for v, slot in seq_t["literals"].items():
+                one[slot] = v
+        for key, n in ins:
+            one[seq[key]:seq[key] + n] = given[key]
+            many[w["L"][key]:w["L"][key] + n] = given[key]
+        one = _in_order(ops, one)
+        assert max(max(op[1:5]) for op in w["ops"]) < w["slots"]
+        looped = _device_loop(ws.encode(w["ops"], w["steps"]), many, ws.LANES)
+        for key, n in outs:
+            want = one[seq[key]:seq[key] + n]
+            assert np.isfinite(want).all() and np.any(want != 0.0)
+            assert np.array_equal(looped[w["L"][key]:w["L"][key] + n], want)
