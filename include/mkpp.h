@@ -151,7 +151,7 @@ size_t mkpp_gpu_workspace_bytes(size_t num_cells);
  * Results do not depend on it: a handed-off cell ends bit-identical. */
 int mkpp_set_launch_tuning(int register_variant, int blocks_per_sm, int defer_after);
 
-/* Process-wide tail parking of the persistent integrate kernel (default 300
+/* Process-wide tail parking of the persistent integrate kernel (default 16
  * attempts, 0: off; environment MKPP_TAIL_AFTER).  Once every cell of a launch has been
  * handed out and no more cells are still on lanes than the warp-cooperative
  * kernel runs at once, a cell with at least min_attempts attempts is parked

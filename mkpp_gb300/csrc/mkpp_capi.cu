@@ -124,15 +124,21 @@ int device_fail(mkpp_handle_s* h, cudaError_t err, const char* what) {
 // Initial values come from MKPP_REGISTER_VARIANT, MKPP_BLOCKS_PER_SM and
 // MKPP_DEFER_AFTER, and mkpp_set_launch_tuning changes them.
 constexpr int kDefaultDeferPerStep = 3000;
-constexpr int kDefaultTailAfter = 300;
+constexpr int kDefaultTailAfter = 16;
 
 struct Tuning {
   int register_variant = 2;
   int blocks_per_sm = 0;
   int defer_after = kDefaultDeferPerStep;
-  // Tail parking threshold in attempts (0: off).  300 measured on SAPRC99:
-  // the 24-step window 38.3 -> 33.6 s, the 24 per-call mkpp_integrate with
-  // cost ordering 218.5 -> 161.7 s, results bit-identical.
+  // Tail parking threshold in attempts (0: off).  Once the queue is drained,
+  // lanes make an attempt per 1-2 ms however few of them still have a cell, so
+  // cells move to the warps as soon as the warps finish them sooner, 16 cells
+  // for each warp of SAPRC99 (attempts before that: 16, the least the kernel
+  // looks at).  65536 cells x 4 host steps: 542 ms, against 575 ms with 8
+  // cells a warp, 624 with 4, 702 with 1, and 815 after 300 attempts; 565 with
+  // all of them.  saprc99_mini, two cells a warp: 14.0 against 16.8 ms without.
+  // Lanes with a register store keep all but the last few (small_strato: 9.6
+  // ms, 10.7 with 10000 cells moved).
   int tail_after = kDefaultTailAfter;
   // Split launch (mkpp_set_split_launch): with a cell order, its first
   // split_cells cells go to whole warps on the first split_sms SMs, the
@@ -152,7 +158,7 @@ struct Tuning {
   // store in registers a few hundred (small_strato: 72 cells 1.8 against 3.1
   // ms, 4096 cells 6.1 against 3.5; Chapman: 0.50 against 0.60 ms, 2.1 against
   // 0.67).
-  int coop_cells = Mech::TABLE_ATTEMPT ? INT32_MAX : Mech::LU_FMA > 2000 ? 40000 : StoreInfo::kTile ? 10000 : 600;
+  int coop_cells = Mech::TABLE_ATTEMPT ? INT32_MAX : Mech::LU_FMA > 2000 ? 20000 : StoreInfo::kTile ? 10000 : 600;
 };
 
 Tuning& tuning() {
@@ -172,14 +178,15 @@ struct LaunchConfig {
   int minb = 0;
   int grid = 0;
   int sms = 0;
+  int warps_per_sm = 0;  // of a mechanism with a register store, whose blocks are single warps
   int coop_per_sm = 0;  // cooperative warps per SM (0: no cooperative kernel)
   bool split_ok = false;
 };
 
 template <int MINB>
-int resident_blocks() {
+int resident_blocks(int threads) {
   int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mkpp::integrate_persistent_kernel<Mech, MINB>, mkpp::kBlock, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mkpp::integrate_persistent_kernel<Mech, MINB>, threads, 0);
   return std::max(1, per_sm);
 }
 
@@ -196,9 +203,11 @@ const LaunchConfig& launch_config() {
     cudaDeviceGetAttribute(&cfg.sms, cudaDevAttrMultiProcessorCount, dev);
     cfg.sms = std::max(1, cfg.sms);
     cfg.minb = t.register_variant;
-    int per_sm = cfg.minb == 4 ? resident_blocks4() : resident_blocks<2>();
+    int per_sm = cfg.minb == 4 ? resident_blocks4() : resident_blocks<2>(mkpp::kBlock);
     if (t.blocks_per_sm > 0) per_sm = std::min(per_sm, t.blocks_per_sm);
     cfg.grid = cfg.sms * per_sm;
+    cfg.warps_per_sm = 4 * per_sm;
+    if (cfg.minb == 2 && t.blocks_per_sm == 0) cfg.warps_per_sm = resident_blocks<2>(32);
     // A cell store larger than a block's shared memory leaves the cooperative
     // kernel unused (no parking).
     cfg.coop_per_sm = coop_resident_blocks(kCoopSmem);
@@ -236,12 +245,55 @@ int launch_rates(size_t cells, const double* conc, const double* temp, const dou
   return cudaGetLastError() == cudaSuccess ? MKPP_SUCCESS : MKPP_ERROR_DEVICE;
 }
 
+// Persistent warps per SM for a call of `cells` cells, of a mechanism whose
+// store fits in registers (one warp per block, so that a small call has a warp
+// on as many SMs as it can).  A warp costs the FP64 pipe the same with one lane
+// at work as with 32, and lanes that finish take new cells one by one, so a
+// pass over the cells ends for all warps at about the same time: with w warps
+// it takes ceil(x / w) rounds of w, x the cells in warps per SM.  The w with
+// the least w * ceil(x / w), six at least to hide latencies (small_strato,
+// 65536 cells, x = 13.5: seven or fourteen instead of eight).
+int persistent_warps(const LaunchConfig& cfg, int cells) {
+  const int x = (int)((cells + 32LL * cfg.sms - 1) / (32LL * cfg.sms));
+  const int most = std::min(x, cfg.warps_per_sm);
+  int best = most;
+  for (int w = most; w >= std::min(6, most); --w)
+    if (w * ((x + w - 1) / w) < best * ((x + best - 1) / best)) best = w;
+  return best;
+}
+
 // Whether the cooperative kernel takes the whole call: few enough cells, and
 // no launch form of the persistent kernel asked for.
 bool coop_alone(const mkpp::LaunchArgs& a) {
   const Tuning& t = tuning();
   return a.ncells <= t.coop_cells && t.defer_after > 0 && t.register_variant == 2 && t.blocks_per_sm == 0 &&
          !(t.split_cells > 0 && a.order);
+}
+
+// Whether a cell order can shorten a call: not when every cell starts at once.
+bool order_pays(size_t cells) {
+  const LaunchConfig& cfg = launch_config();
+  mkpp::LaunchArgs a = {};
+  a.ncells = (int)cells;
+  if (cfg.coop_per_sm > 0 && coop_alone(a)) return cells > (size_t)cfg.sms * cfg.coop_per_sm;
+  return cells > (StoreInfo::kTile ? (size_t)cfg.grid * mkpp::kBlock : (size_t)cfg.sms * cfg.warps_per_sm * 32);
+}
+
+// Cells by attempts of the previous call, most first; ties keep the cell
+// order.  By counting (40000 cells: 0.1 ms, a comparison sort 2 ms).
+void sort_by_cost(const std::vector<int>& cost, std::vector<int>& order) {
+  const size_t n = cost.size();
+  order.resize(n);
+  const int most = *std::max_element(cost.begin(), cost.end());
+  if (most >= 1 << 20) {
+    for (size_t c = 0; c < n; ++c) order[c] = (int)c;
+    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cost[x] > cost[y]; });
+    return;
+  }
+  std::vector<int> at(most + 2, 0);  // at[most - cost]: the next position of that cost
+  for (size_t c = 0; c < n; ++c) ++at[most - cost[c] + 1];
+  for (int v = 0; v <= most; ++v) at[v + 1] += at[v];
+  for (size_t c = 0; c < n; ++c) order[at[most - cost[c]]++] = (int)c;
 }
 
 int launch_integrate(const mkpp::LaunchArgs& args, int mode, void* workspace, cudaStream_t stream) {
@@ -275,18 +327,20 @@ int launch_integrate(const mkpp::LaunchArgs& args, int mode, void* workspace, cu
     a.defer_after = (int)std::min<long long>(park, INT32_MAX);
     // Tail parking runs in the 255-register variant only.
     const bool tail = t.tail_after > 0 && cfg.minb == 2;
+    const int threads = StoreInfo::kTile ? mkpp::kBlock : 32;
+    const int grid = StoreInfo::kTile ? cfg.grid : cfg.sms * persistent_warps(cfg, a.ncells);
     a.defer = (a.defer_after > 0 || tail) && coop_blocks > 0 ? (mkpp::Deferred*)(ws + defer_offset()) : nullptr;
     if (!a.defer) a.defer_after = 0;
     if (tail && a.defer) {
       a.tail_after = t.tail_after;
-      a.tail_cells = (unsigned)coop_blocks;
-      if (launch_persistent_tail(a, scratch, cfg.grid, stream) != MKPP_SUCCESS) return MKPP_ERROR_DEVICE;
+      a.tail_cells = (unsigned)(StoreInfo::kTile ? coop_blocks * (Mech::LU_FMA > 2000 ? 16 : 2) : cfg.sms);
+      if (launch_persistent_tail(a, scratch, grid, threads, stream) != MKPP_SUCCESS) return MKPP_ERROR_DEVICE;
     } else if (split) {
       if (launch_split(a, scratch, cfg.grid, stream) != MKPP_SUCCESS) return MKPP_ERROR_DEVICE;
     } else if (cfg.minb == 4) {
-      if (launch_persistent4(a, scratch, cfg.grid, stream) != MKPP_SUCCESS) return MKPP_ERROR_DEVICE;
+      if (launch_persistent4(a, scratch, grid, threads, stream) != MKPP_SUCCESS) return MKPP_ERROR_DEVICE;
     } else {
-      mkpp::integrate_persistent_kernel<Mech, 2><<<cfg.grid, mkpp::kBlock, 0, stream>>>(a, scratch);
+      mkpp::integrate_persistent_kernel<Mech, 2><<<grid, threads, 0, stream>>>(a, scratch);
     }
     if (a.defer) {
       if (launch_coop(a, coop_blocks, kCoopSmem, stream) != MKPP_SUCCESS) {
@@ -599,11 +653,9 @@ int mkpp_integrate(mkpp_handle_t handle, double dt) {
   const size_t n = h->num_cells;
   mkpp::LaunchArgs args = make_args(n, d.conc, d.ktab, 1, dt, h->seed, h->max_attempts, d.status, d.accepted,
                                     d.rejected);
-  if (h->cost_order && h->cost.size() == n) {
-    // Most expensive first; ties keep the cell order.
-    h->order.resize(n);
-    for (size_t c = 0; c < n; ++c) h->order[c] = (int)c;
-    std::stable_sort(h->order.begin(), h->order.end(), [h](int x, int y) { return h->cost[x] > h->cost[y]; });
+  const bool cost_order = h->cost_order && order_pays(n);
+  if (cost_order && h->cost.size() == n) {
+    sort_by_cost(h->cost, h->order);
     if (!d.order) MKPP_CUDA(h, cudaMalloc(&d.order, n * sizeof(int)));
     MKPP_CUDA(h, cudaMemcpyAsync(d.order, h->order.data(), n * sizeof(int), cudaMemcpyHostToDevice, h->stream));
     args.order = d.order;
@@ -621,7 +673,7 @@ int mkpp_integrate(mkpp_handle_t handle, double dt) {
   if (rc != MKPP_SUCCESS) return device_fail(h, cudaGetLastError(), "integrate kernel launch");
   MKPP_CUDA(h, cudaMemcpyAsync(h->conc, d.conc, n * Mech::NS * sizeof(double), cudaMemcpyDeviceToHost,
                                h->stream));
-  if (h->cost_order) {
+  if (cost_order) {
     h->cost.resize(n);
     h->rejected.resize(n);
     MKPP_CUDA(h, cudaMemcpyAsync(h->cost.data(), d.accepted, n * sizeof(int), cudaMemcpyDeviceToHost, h->stream));
@@ -629,7 +681,7 @@ int mkpp_integrate(mkpp_handle_t handle, double dt) {
                                  h->stream));
   }
   MKPP_CUDA(h, cudaStreamSynchronize(h->stream));
-  if (h->cost_order)
+  if (cost_order)
     for (size_t c = 0; c < n; ++c) h->cost[c] += h->rejected[c];
   return MKPP_SUCCESS;
 }

@@ -61,6 +61,73 @@ struct KLocal {
 
 __device__ __forceinline__ bool finite(double x) { return isfinite(x); }
 
+__device__ __forceinline__ bool is_zero(double x) { return (__double_as_longlong(x) << 1) == 0; }
+
+// ---------------------------------------------------------------------------
+// a / b, correctly rounded, in 32-bit integer arithmetic.
+//
+// The FP64 pipe of GB300 issues a warp instruction per 64 cycles and a
+// division takes it six to nine of them, half of a small mechanism's attempt
+// (Chapman: 12 divisions); the integer pipes are idle.  Long division in base
+// 2^28: with the significands n and d as integers and X an underestimate of
+// 2^62 / (d / 2^22) to 2^-30 (the hardware's FP32 reciprocal and one Newton
+// step), two quotient digits (n X, then R X of the remainder) give 56 bits that
+// are at most 2 short, which the remainder corrects; the rest is rounding to
+// nearest even with the remainder as the sticky bit.  Exponents outside the
+// normal range, on either side or in the result, take the hardware's division.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ double divide(double a, double b) {
+#ifdef __CUDA_ARCH__
+  typedef unsigned long long u64;
+  const u64 ab = (u64)__double_as_longlong(a), bb = (u64)__double_as_longlong(b);
+  const int ea = (int)(ab >> 52) & 0x7ff, eb = (int)(bb >> 52) & 0x7ff;
+  const int e = ea - eb + 1023;
+  constexpr u64 kOne = 1ull << 52;
+  const bool zero = is_zero(a);
+  if ((unsigned)(eb - 1) >= 2046u || (!zero && ((unsigned)(ea - 1) >= 2046u || (unsigned)(e - 2) >= 2043u)))
+    return a / b;
+  const u64 n = (ab & (kOne - 1)) | kOne, d = (bb & (kOne - 1)) | kOne;
+  const unsigned D = (unsigned)(d >> 22) + 1u;  // at most 2^31
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(__uint2float_rn(D)));
+  const unsigned X0 = __float2uint_rz(r * 4.6116838e18f);  // 2^62 (1 - 2^-21): below 2^62 / D
+  const u64 short_of = (1ull << 62) - (u64)X0 * D;         // below 2^42
+  const unsigned X = X0 + (unsigned)(((u64)X0 * (unsigned)(short_of >> 10)) >> 52);
+  const unsigned q1 = (unsigned)(((u64)(unsigned)(n >> 21) * X) >> 36);
+  u64 R = (n << 27) - q1 * d;                              // below 2^55
+  const unsigned q2 = (unsigned)(((u64)(unsigned)(R >> 23) * X) >> 33);
+  R = (R << 28) - q2 * d;                                  // below 3 d
+  u64 q = ((u64)q1 << 28) + q2;
+  if (R >= 2 * d) {
+    R -= 2 * d;
+    q += 2;
+  }
+  if (R >= d) {
+    R -= d;
+    q += 1;
+  }
+  q |= R != 0;
+  // q is n / d * 2^55: 56 bits where n >= d, else 55.
+  const unsigned top = (unsigned)(q >> 55);
+  const unsigned drop = 2u + top;
+  const u64 m = (q + ((1u << (drop - 1)) - 1u) + ((q >> drop) & 1u)) >> drop;
+  const u64 bits = ((u64)(unsigned)(e - 2 + (int)top) << 52) + m;  // m's leading bit adds one to the exponent
+  const u64 sign = (ab ^ bb) & (1ull << 63);
+  return __longlong_as_double((long long)((zero ? 0ull : bits) | sign));
+#else
+  return a / b;
+#endif
+}
+
+// fmax(fabs(x), fabs(y)) by the bit patterns, off the FP64 pipe.
+__device__ __forceinline__ double max_abs(double x, double y) {
+  const unsigned long long mask = ~(1ull << 63), inf = 0x7ffull << 52;
+  const unsigned long long ax = (unsigned long long)__double_as_longlong(x) & mask;
+  const unsigned long long ay = (unsigned long long)__double_as_longlong(y) & mask;
+  const bool take_y = ax > inf || (ay <= inf && ay > ax);
+  return __longlong_as_double((long long)(take_y ? ay : ax));
+}
+
 // ---------------------------------------------------------------------------
 // Programs of uniform operations S[out] = fma(+-S[a], S[b], S[c]) or
 // S[out] = 1 / S[b], one 64-bit word each, four 16-bit fields of slot * 4 plus
@@ -85,7 +152,6 @@ struct ProgramWord {
 __device__ __forceinline__ double flip_sign(double x, unsigned sign) {
   return __longlong_as_double(__double_as_longlong(x) ^ ((long long)sign << 32));
 }
-__device__ __forceinline__ bool is_zero(double x) { return (__double_as_longlong(x) << 1) == 0; }
 
 // Sequential form: one thread runs `ops` words on its own store.  Returns
 // false if a reciprocal met a zero.
@@ -98,7 +164,7 @@ __device__ __forceinline__ bool run_program(SA& S, const unsigned long long* __r
     const double B = w.prev_b() ? prev : S[w.b()];
     if (w.reciprocal()) {
       ok = ok && !is_zero(B);
-      prev = 1.0 / B;
+      prev = divide(1.0, B);
     } else {
       const double C = w.prev_c() ? prev : S[w.c()];
       prev = fma(flip_sign(S[w.a()], w.negate()), B, C);

@@ -10,8 +10,9 @@ int resident_blocks4() {
   return std::max(1, per_sm);
 }
 
-int launch_persistent4(const mkpp::LaunchArgs& a, double* scratch, int grid, cudaStream_t stream) {
-  mkpp::integrate_persistent_kernel<Mech, 4><<<grid, mkpp::kBlock, 0, stream>>>(a, scratch);
+int launch_persistent4(const mkpp::LaunchArgs& a, double* scratch, int grid, int threads,
+                           cudaStream_t stream) {
+  mkpp::integrate_persistent_kernel<Mech, 4><<<grid, threads, 0, stream>>>(a, scratch);
   return cudaGetLastError() == cudaSuccess ? MKPP_SUCCESS : MKPP_ERROR_DEVICE;
 }
 

@@ -6,8 +6,9 @@
 
 namespace mkpp_tu {
 
-int launch_persistent_tail(const mkpp::LaunchArgs& a, double* scratch, int grid, cudaStream_t stream) {
-  mkpp::integrate_persistent_kernel<Mech, 2, true><<<grid, mkpp::kBlock, 0, stream>>>(a, scratch);
+int launch_persistent_tail(const mkpp::LaunchArgs& a, double* scratch, int grid, int threads,
+                           cudaStream_t stream) {
+  mkpp::integrate_persistent_kernel<Mech, 2, true><<<grid, threads, 0, stream>>>(a, scratch);
   return cudaGetLastError() == cudaSuccess ? MKPP_SUCCESS : MKPP_ERROR_DEVICE;
 }
 

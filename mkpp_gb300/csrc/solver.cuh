@@ -142,6 +142,12 @@ __global__ void __launch_bounds__(128) rate_constant_kernel(RateArgs a) {
 // ---------------------------------------------------------------------------
 constexpr int kBlock = 128;
 constexpr int kRegisterSlots = 96;
+struct TileStore;
+// Unroll factor of a loop over n slots: a store in registers needs constant
+// indices (small_strato has ten rate constants; unrolled by eight they put its whole
+// store into local memory).
+template <class Store, int N, int Tile>
+constexpr int slot_unroll = std::is_same<Store, TileStore>::value ? Tile : N;
 
 template <int N>
 struct RegStore {
@@ -258,7 +264,7 @@ template <class Mech, class SA>
 __device__ __forceinline__ void load_rates(const LaunchArgs& a, size_t c, int step, SA& S) {
   const double* __restrict__ k = a.ktab + (size_t)step * a.k_step_stride + c;
   const size_t n = (size_t)a.ncells;
-#pragma unroll 8
+#pragma unroll(slot_unroll<SA, Mech::NR, 8>)
   for (int r = 0; r < Mech::NR; ++r) S[Mech::KT + r] = __ldg(k + (size_t)r * n);
 }
 
@@ -710,7 +716,7 @@ __global__ void __launch_bounds__(kBlock, 2) integrate_checkpoint_kernel(LaunchA
           overflow = true;
           break;
         }
-#pragma unroll 4
+#pragma unroll(slot_unroll<typename SN::type, Mech::NV, 4>)
         for (int i = 0; i < Mech::NV; ++i) ck.y[((size_t)cnt * Mech::NV + i) * n + c] = S[Mech::Y + i];
         ck.h[(size_t)cnt * n + c] = h;
         ++cnt;
@@ -769,16 +775,16 @@ __global__ void __launch_bounds__(kBlock, 2) adjoint_kernel(AdjointArgs a, Check
   const size_t n = (size_t)a.ncells;
   const size_t T = (size_t)gridDim.x * kBlock;
   for (size_t c = blockIdx.x * (size_t)kBlock + threadIdx.x; c < n; c += T) {
-#pragma unroll 4
+#pragma unroll(slot_unroll<typename SN::type, Mech::NR, 4>)
     for (int r = 0; r < Mech::NR; ++r) {
       S[Mech::KT + r] = __ldg(a.ktab + (size_t)r * n + c);
       S[Mech::KB + r] = 0.0;
     }
-#pragma unroll 4
+#pragma unroll(slot_unroll<typename SN::type, Mech::NV, 4>)
     for (int i = 0; i < Mech::NV; ++i) S[Mech::LAM + i] = a.lam[c + n * Mech::var_phys(i)];
     auto k = [&](int r) { return S[Mech::KT + r]; };
     for (int s = ck.count(c) - 1; s >= 0; --s) {
-#pragma unroll 4
+#pragma unroll(slot_unroll<typename SN::type, Mech::NV, 4>)
       for (int i = 0; i < Mech::NV; ++i) S[Mech::Y + i] = ck.y[((size_t)s * Mech::NV + i) * n + c];
       const double h = ck.h[(size_t)s * n + c];
       int st = 0;
@@ -786,9 +792,9 @@ __global__ void __launch_bounds__(kBlock, 2) adjoint_kernel(AdjointArgs a, Check
       Mech::adjoint_step(S, k, h);
     }
     for (int i = 0; i < Mech::NS; ++i) a.grad_conc[c + n * i] = 0.0;
-#pragma unroll 4
+#pragma unroll(slot_unroll<typename SN::type, Mech::NV, 4>)
     for (int i = 0; i < Mech::NV; ++i) a.grad_conc[c + n * Mech::var_phys(i)] = S[Mech::LAM + i];
-#pragma unroll 4
+#pragma unroll(slot_unroll<typename SN::type, Mech::NR, 4>)
     for (int r = 0; r < Mech::NR; ++r) a.grad_k[c + n * r] = S[Mech::KB + r];
   }
 }

@@ -59,7 +59,7 @@ struct WarpProgram {
         if constexpr (decltype(pivots)::value) {
           if (__any_sync(0xffffffffu, p.reciprocal())) {
             ok = ok && !(p.reciprocal() && is_zero(b));
-            const double r = 1.0 / (p.reciprocal() ? b : 1.0);
+            const double r = divide(1.0, p.reciprocal() ? b : 1.0);
             v = p.reciprocal() ? r : v;
           }
         }

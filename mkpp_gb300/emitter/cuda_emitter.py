@@ -760,7 +760,7 @@ def _emit_tlm(c, t, tlm, C):
     c("    for (int i = 0; i < TLM_NCONST; ++i) S[TLM_CB + i] = coop::tlm_const_val[i];")
     for (st, j), slot in tlm["cterm"].items():
         cv = C[(st - 1) * (st - 2) // 2 + j - 1]
-        c(f"    S[{slot}] = {_lit(cv)} / h;    // c{st}{j} / h")
+        c(f"    S[{slot}] = mkpp::divide({_lit(cv)}, h);    // c{st}{j} / h")
     c("    mkpp::run_program(S, coop::tlm_prog, coop::TLM_OPS);")
     c("  }")
 
@@ -812,10 +812,10 @@ def _emit_table_attempt_head(c, coop, C):
     c("  __device__ __forceinline__ static double attempt(SA& S, const KA& k, double h, int& status) {")
     c("    for (int r = 0; r < NR; ++r) S[KT + r] = k(r);")
     c("    for (int i = 0; i < NCONST; ++i) S[CB + i] = coop::const_val[i];")
-    c("    S[CB + 3] = 1.0 / (GAMMA * h);")
+    c("    S[CB + 3] = mkpp::divide(1.0, GAMMA * h);")
     for (st, j), slot in coop["cterm_slot"].items():
         cv = C[(st - 1) * (st - 2) // 2 + j - 1]
-        c(f"    S[{slot}] = {_lit(cv)} / h;    // c{st}{j} / h")
+        c(f"    S[{slot}] = mkpp::divide({_lit(cv)}, h);    // c{st}{j} / h")
     c("    if (!mkpp::run_program(S, coop::attempt_prog, coop::ATTEMPT_OPS)) status |= 1;")
 
 
@@ -893,7 +893,7 @@ def _emit_coop(c, plan, coop, nv, ns, stages, C, M, E, K0, Y, FS, DY):
     c("                                                    const Run& run) {")
     c("    namespace T = coop;")
     c("    // 1/(gamma h) and the c_ij/h, one division of the whole warp.")
-    c("    if (lane < T::H_TERMS) S[WCB + 3 + lane] = T::h_num[lane] / (lane == 0 ? GAMMA * h : h);")
+    c("    if (lane < T::H_TERMS) S[WCB + 3 + lane] = mkpp::divide(T::h_num[lane], lane == 0 ? GAMMA * h : h);")
     c("    __syncwarp();")
     c("    const bool ok = run(S, T::sched, T::stage_step[NSTAGE], lane);")
     c("    if (__any_sync(0xffffffffu, !ok)) status |= 1;")
@@ -927,14 +927,14 @@ def _emit_coop(c, plan, coop, nv, ns, stages, C, M, E, K0, Y, FS, DY):
         ynew = f"{ynew} + k{j}" if cv == 1.0 else f"fma({_lit(cv)}, k{j}, {ynew})"
     c(f"      const double ynew = {ynew};")
     c(f"      S[DY + i] = {lin(mterms)};")
-    c("      const double sc = fma(rtol_v(i), fmax(fabs(yi), fabs(ynew)), atol_v(i));")
-    c(f"      S[Q + i] = ({lin(eterms)}) / sc;")
+    c("      const double sc = fma(rtol_v(i), mkpp::max_abs(yi, ynew), atol_v(i));")
+    c(f"      S[Q + i] = mkpp::divide({lin(eterms)}, sc);")
     c("    }")
     c("    __syncwarp();")
     c("    double err_sq = 0.0;")
     c("    #pragma unroll 8")
     c("    for (int i = 0; i < NV; ++i) err_sq = fma(S[Q + i], S[Q + i], err_sq);")
-    c(f"    return fmax(sqrt(err_sq / {ns}.0), 1.0e-10);")
+    c(f"    return fmax(sqrt(mkpp::divide(err_sq, {ns}.0)), 1.0e-10);")
     c("  }")
     for line in tlm_code.lines:
         c(line)
@@ -1192,7 +1192,7 @@ def _emit_adjoint(c, plan, nv, nr, stages, A, C, M, NewF, K0, Y, nslots):
         for j in range(i):
             cv = C[i * (i - 1) // 2 + j]
             if cv != 0.0:
-                c(f"    {{ const double cc = {_lit(cv)} / h;")
+                c(f"    {{ const double cc = mkpp::divide({_lit(cv)}, h);")
                 c("      #pragma unroll")
                 c(f"      for (int q = 0; q < NV; ++q) S[KBAR + {j * nv} + q] = fma(cc, S[{kb_i} + q], S[KBAR + {j * nv} + q]); }}")
         if NewF[i]:
@@ -1372,6 +1372,10 @@ def emit_mechanism(plan: ReducedPlan, table: bool | None = None) -> str:
     # stores stay inlined, since a call would move them to local memory.
     store_slots = coop["total"] if table else nslots
     fn_inline = "__noinline__" if store_slots > REGISTER_SLOTS else "__forceinline__"
+    # Divisions of the per-thread code: in integers for register stores.  With
+    # the store in the global tile the unrolled attempt has 160 of them, 70
+    # instructions each, and lost 6% (SAPRC99, 65536 cells x 4 host steps).
+    div = "mkpp::divide({}, {})" if store_slots <= REGISTER_SLOTS else "{} / {}"
     # ---------------- Fun
     used_y_f = sorted({v2l[s_] for r in plan.reactions for s_, _ in r.reactants})
     c("  // Mass-action tendencies F(y) of the variable species (logical order):")
@@ -1508,8 +1512,8 @@ def emit_mechanism(plan: ReducedPlan, table: bool | None = None) -> str:
                 l_, u_ = plan.products[q]
                 expr = f"fma(-a{l_}, S[{u_}], {expr})"
             c(f"      const double u{out} = {expr};")
-            c(f"      ok = ok && (u{out} != 0.0);")
-            c(f"      const double rd = 1.0 / u{out};")
+            c(f"      ok = ok && !mkpp::is_zero(u{out});")
+            c(f"      const double rd = {div.format('1.0', f'u{out}')};")
             c(f"      S[{out}] = rd;")
         _interleave(c, plan, rest_u, lambda q: (f"a{plan.products[q][0]}", f"S[{plan.products[q][1]}]"), None)
         uslots = sorted({plan.products[q][1] for o in lpart for q in range(o[2], o[3])})
@@ -1544,7 +1548,7 @@ def emit_mechanism(plan: ReducedPlan, table: bool | None = None) -> str:
     c("  // Bit 1 of status is set on a zero pivot.")
     c("  template <class SA, class KA>")
     c("  __device__ __forceinline__ static double attempt(SA& S, const KA& k, double h, int& status) {")
-    c("    const double inv_g_dt = 1.0 / (GAMMA * h);")
+    c(f"    const double inv_g_dt = {div.format('1.0', '(GAMMA * h)')};")
     c("    jac_w([&](int i) { return S[Y + i]; }, k, inv_g_dt, S);")
     c("    if (!factor(S)) status |= 1;")
     for st in range(1, stages + 1):
@@ -1570,7 +1574,7 @@ def emit_mechanism(plan: ReducedPlan, table: bool | None = None) -> str:
                 if cv != 0.0:
                     cterms.append((cv, j))
         for cv, j in cterms:
-            c(f"    const double c{st}{j} = {_lit(cv)} / h;")
+            c(f"    const double c{st}{j} = {div.format(_lit(cv), 'h')};")
         c("    #pragma unroll")
         c("    for (int i = 0; i < NV; ++i) {")
         expr = "S[F + i]"
@@ -1608,19 +1612,19 @@ def emit_mechanism(plan: ReducedPlan, table: bool | None = None) -> str:
         ynew = f"{ynew} + k{j}" if cv == 1.0 else f"fma({_lit(cv)}, k{j}, {ynew})"
     c(f"      const double ynew = {ynew};")
     c(f"      S[DY + i] = {lin(mterms)};")
-    c("      const double sc = fma(rtol_v(i), fmax(fabs(yi), fabs(ynew)), atol_v(i));")
-    c(f"      const double q = ({lin(eterms)}) / sc;")
+    c("      const double sc = fma(rtol_v(i), mkpp::max_abs(yi, ynew), atol_v(i));")
+    c(f"      const double q = {div.format('(' + lin(eterms) + ')', 'sc')};")
     c("      err_sq = fma(q, q, err_sq);")
     c("    }")
-    c(f"    return fmax(sqrt(err_sq / {ns}.0), 1.0e-10);")
+    c(f"    return fmax(sqrt(mkpp::divide(err_sq, {ns}.0)), 1.0e-10);")
     c("  }")
     c("")
     c("  // Step-size factor from the error norm (integrate.j2:324-333).")
     c("  __device__ __forceinline__ static double growth(double err) {")
     if elo == 2.0:
-        c("    const double fac = 0.9 / sqrt(err);")
+        c("    const double fac = mkpp::divide(0.9, sqrt(err));")
     elif elo == 3.0:
-        c("    const double fac = 0.9 / cbrt(err);")
+        c("    const double fac = mkpp::divide(0.9, cbrt(err));")
     else:
         c(f"    const double fac = 0.9 * pow(err, -{_lit(1.0 / elo)});")
     c("    return fmax(0.2, fmin(fac, 6.0));")
