@@ -575,8 +575,8 @@ def main():
     lib = load_library(w.mechanism)
     solver = DeviceSolver(w.mechanism)
     # Tail parking threshold the runs use unless the tuning below picks
-    # another: the flag, else the library's default (MKPP_TAIL_AFTER or 300).
-    lib_tail = args.tail_after if args.tail_after is not None else int(os.environ.get("MKPP_TAIL_AFTER", "300"))
+    # another: the flag, else the library's default (MKPP_TAIL_AFTER or 16).
+    lib_tail = args.tail_after if args.tail_after is not None else int(os.environ.get("MKPP_TAIL_AFTER", "16"))
     solver.set_tail_parking(lib_tail)
     NS, NR, NP = solver.sizes.species, solver.sizes.reactions, solver.sizes.rate_parameters
     seed = float(raw["initial_step_seed"])
@@ -629,8 +629,8 @@ def main():
     # gives every cell's attempt count; each later warm-up window (now in
     # cost order) runs one candidate launch configuration, and the fastest
     # is the one timed:
-    #   default   the library's settings (tail parking after 300 attempts);
-    #   tail      tail parking after 300 attempts, where the flags turned it
+    #   default   the library's settings (tail parking after 16 attempts);
+    #   tail      tail parking after 16 attempts, where the flags turned it
     #             off (mkpp_set_tail_parking);
     #   split     the split launch (mkpp_set_split_launch): the 0.1% most
     #             expensive cells of the previous window on whole warps of
@@ -655,7 +655,7 @@ def main():
     configs = [{"name": "default", "tail": lib_tail, "split": (0, 0) if tune_info["tuned"] else fixed_split}]
     if tune_info["tuned"]:
         if lib_tail == 0:
-            configs.append({"name": "tail", "tail": 300, "split": (0, 0)})
+            configs.append({"name": "tail", "tail": 16, "split": (0, 0)})
         if args.split != "off":
             configs.append({"name": "split", "tail": 0, "split": auto_split})
     ev = (torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True))

@@ -40,7 +40,7 @@ __global__ void __launch_bounds__(32) checkpoint_coop_kernel(LaunchArgs a, Check
       }
       const double h = ctl.next_h();
       int st = 0;
-      const double err = Mech::attempt_coop(S, h, st, lane, WarpProgram());
+      const double err = Mech::attempt_coop(S, h, st, lane, WarpProgram<Mech::PIVOT_EVERY>());
       zero_pivot |= st != 0;
       if (ctl.update<Mech>(err)) {
         if (cnt >= ck.cap) {
@@ -97,8 +97,8 @@ __global__ void __launch_bounds__(32) adjoint_coop_kernel(AdjointArgs a, Checkpo
       for (int i = lane; i < Mech::NV; i += 32) S[Mech::Y + i] = ck.y[((size_t)s * Mech::NV + i) * n + c];
       __syncwarp();
       int st = 0;
-      Mech::stages_coop(S, ck.h[(size_t)s * n + c], st, lane, WarpProgram());
-      Mech::adjoint_coop(S, lane, WarpProgram());
+      Mech::stages_coop(S, ck.h[(size_t)s * n + c], st, lane, WarpProgram<Mech::PIVOT_EVERY>());
+      Mech::adjoint_coop(S, lane, WarpProgram<Mech::PIVOT_EVERY>());
     }
     for (int i = lane; i < Mech::NS; i += 32) a.grad_conc[c + n * i] = 0.0;
     __syncwarp();
@@ -130,8 +130,8 @@ __global__ void __launch_bounds__(32) tangent_coop_kernel(TangentArgs a, Checkpo
       for (int i = lane; i < Mech::NV; i += 32) S[Mech::Y + i] = ck.y[((size_t)s * Mech::NV + i) * n + c];
       __syncwarp();
       int st = 0;
-      Mech::stages_coop(S, ck.h[(size_t)s * n + c], st, lane, WarpProgram());
-      Mech::tangent_coop(S, lane, WarpProgram());
+      Mech::stages_coop(S, ck.h[(size_t)s * n + c], st, lane, WarpProgram<Mech::PIVOT_EVERY>());
+      Mech::tangent_coop(S, lane, WarpProgram<Mech::PIVOT_EVERY>());
     }
     for (int i = lane; i < Mech::NS; i += 32) a.dconc[c + n * i] = 0.0;
     __syncwarp();

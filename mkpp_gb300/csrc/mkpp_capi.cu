@@ -158,7 +158,7 @@ struct Tuning {
   // store in registers a few hundred (small_strato: 72 cells 1.8 against 3.1
   // ms, 4096 cells 6.1 against 3.5; Chapman: 0.50 against 0.60 ms, 2.1 against
   // 0.67).
-  int coop_cells = Mech::TABLE_ATTEMPT ? INT32_MAX : Mech::LU_FMA > 2000 ? 20000 : StoreInfo::kTile ? 10000 : 600;
+  int coop_cells = Mech::TABLE_ATTEMPT ? INT32_MAX : Mech::LU_FMA > 2000 ? 14000 : StoreInfo::kTile ? 10000 : 600;
 };
 
 Tuning& tuning() {

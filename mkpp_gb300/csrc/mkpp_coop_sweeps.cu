@@ -26,16 +26,16 @@ constexpr size_t kSlots = std::max(std::max(Mech::WARP_SLOTS, Mech::ADJ_COOP_SLO
 
 }  // namespace
 
-// Up to half the cells of a plain integrate: the sweeps' stores are larger, and
-// both forms spend about twice the operations per step.  small_strato's and
-// saprc99_mini's sweeps gain longer, as their lanes keep more slots than
-// registers hold: 2000 cells 7.3 against 9.8 ms (gradient) and 7.4 against 19
-// ms (tangent), 16384 cells 41 against 10 ms; saprc99_mini, 8192 cells 6.1
-// against 9.4 ms.
-bool sweep_on_warps(size_t cells) {
-  constexpr size_t kLeast = Mech::NLU > 20 ? (StoreInfo::kTile ? 10000 : 2000) : 0;
-  return kSlots * sizeof(double) <= kMaxSmem && coop_cells() > 0 &&
-         cells <= std::max((size_t)coop_cells() / 2, kLeast);
+// Up to as many cells as a plain integrate, whose lanes take half as long per
+// step; small_strato's tangent, whose lanes walk a program on the global tile,
+// up to more (4325 cells: 11.6 against 15 ms, 8000: 19 against 15; its gradient
+// 11.3 against 9.7 ms, 2000 cells 6.3 against 6.6).
+bool sweep_on_warps(size_t cells, bool tangent) {
+  constexpr size_t kRegister = Mech::NLU > 20 ? 2000 : 300, kTangent = Mech::NLU > 20 ? 5000 : 300;
+  const size_t most = coop_cells() == 0 ? 0
+                      : StoreInfo::kTile ? (size_t)coop_cells()
+                                         : (tangent ? kTangent : kRegister);
+  return kSlots * sizeof(double) <= kMaxSmem && cells <= most;
 }
 
 int launch_checkpoint_coop(mkpp::LaunchArgs a, const mkpp::CheckpointArgs& ck, unsigned* next, cudaStream_t stream) {

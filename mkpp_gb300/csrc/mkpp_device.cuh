@@ -153,21 +153,32 @@ __device__ __forceinline__ double flip_sign(double x, unsigned sign) {
   return __longlong_as_double(__double_as_longlong(x) ^ ((long long)sign << 32));
 }
 
-// Sequential form: one thread runs `ops` words on its own store.  Returns
-// false if a reciprocal met a zero.
-template <class SA>
+// Sequential form: one thread runs `ops` words on its own store.  Bound by the
+// latency of a word's operands, so those of the next word are loaded before
+// this one's result is stored (what it reads of that comes from the register).
+// Returns false if a reciprocal met a zero; a program without pivots says so,
+// which keeps the division out of its loop.
+template <bool kPivots, class SA>
 __device__ __forceinline__ bool run_program(SA& S, const unsigned long long* __restrict__ prog, int ops) {
   double prev = 0.0;
   bool ok = true;
+  unsigned long long now = __ldg(prog), next = __ldg(prog + (ops > 1 ? 1 : 0));
+  double A = S[ProgramWord(now).a()], B = S[ProgramWord(now).b()], C = S[ProgramWord(now).c()];
+#pragma unroll 4
   for (int n = 0; n < ops; ++n) {
-    const ProgramWord w(__ldg(prog + n));
-    const double B = w.prev_b() ? prev : S[w.b()];
-    if (w.reciprocal()) {
-      ok = ok && !is_zero(B);
-      prev = divide(1.0, B);
-    } else {
-      const double C = w.prev_c() ? prev : S[w.c()];
-      prev = fma(flip_sign(S[w.a()], w.negate()), B, C);
+    const ProgramWord w(now), following(next);
+    now = next;
+    next = __ldg(prog + (n + 2 < ops ? n + 2 : ops - 1));
+    const double a = flip_sign(A, w.negate()), b = w.prev_b() ? prev : B, c = w.prev_c() ? prev : C;
+    A = S[following.a()];
+    B = S[following.b()];
+    C = S[following.c()];
+    prev = fma(a, b, c);
+    if constexpr (kPivots) {
+      if (w.reciprocal()) {
+        ok = ok && !is_zero(b);
+        prev = divide(1.0, b);
+      }
     }
     if (w.stores()) S[w.out()] = prev;
   }

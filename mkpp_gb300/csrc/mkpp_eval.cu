@@ -5,13 +5,13 @@
 // with the arithmetic of fun() and jac_w().
 //
 // Both are bound by memory: the Jacobian is NS^2 values per cell written once.
-// A block takes 32 cells, one per lane, and its warps share their rates (or
-// one column's partial derivatives) in shared memory and divide the rows, so
+// A block takes 32 cells, one per lane (64 for the Jacobian), and its warps
+// share their rates (or one column's partial derivatives) in shared memory and divide the rows, so
 // that every output row is one coalesced store per warp and a small call
 // still has blocks for all SMs.  A thread per cell, which zero-filled the
 // matrix, wrote W and flipped its sign through tables of slot positions on the
-// stack, took 92.8 ms for SAPRC99's 20000 cells (1.08 GB); this takes 0.26 ms.
-// TS1, 1001 cells: 4.5 -> 0.10 ms, the tendencies 3.1 -> 0.08 ms.
+// stack, took 92.8 ms for SAPRC99's 20000 cells (1.08 GB); this takes 0.23 ms.
+// TS1, 1001 cells: 4.5 -> 0.11 ms, the tendencies 3.1 -> 0.06 ms.
 #include "capi_common.cuh"
 
 using namespace mkpp_tu;
@@ -20,9 +20,9 @@ namespace {
 
 namespace T = MKPP_MECH_NS::eval;
 
-constexpr int kWarps = 8;
+constexpr int kWarps = 8;       // of a block, one column of the Jacobian
+constexpr int kRateWarps = 16;  // of a block, all rates and tendencies
 constexpr size_t kRatesSmem = (size_t)Mech::NR * 32 * sizeof(double);
-constexpr size_t kJacSmem = (size_t)(T::MAX_PARTIALS > 0 ? T::MAX_PARTIALS : 1) * 32 * sizeof(double);
 constexpr size_t kDefaultSmem = 48 * 1024;
 
 // State accessor over a cell's row of the (species x cells) array.
@@ -72,49 +72,89 @@ __device__ __forceinline__ double product(double k, unsigned code, const double*
   return v;
 }
 
-__global__ void __launch_bounds__(kWarps * 32) eval_rates_kernel(size_t n, const double* __restrict__ conc,
+// c * t; most coefficients are 1 or -1, which cost no FP64 instruction.
+__device__ __forceinline__ double first_term(double c, double t) {
+  const long long bits = __double_as_longlong(c);
+  return (bits << 1) == (__double_as_longlong(1.0) << 1) ? mkpp::flip_sign(t, (unsigned)(bits >> 32) & 0x80000000u)
+                                                         : c * t;
+}
+
+__global__ void __launch_bounds__(kRateWarps * 32) eval_rates_kernel(size_t n, const double* __restrict__ conc,
                                                                 const double* __restrict__ ktab,
                                                                 double* __restrict__ out) {
   extern __shared__ double q[];  // [reaction][lane]
   const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const size_t cell = blockIdx.x * (size_t)32 + lane;
   const size_t c = cell < n ? cell : n - 1;
-  for (int r = warp; r < Mech::NR; r += kWarps)
+  for (int r = warp; r < Mech::NR; r += kRateWarps)
     q[r * 32 + lane] = product(__ldg(ktab + c + n * r), T::rate[r], conc, c, n);
   __syncthreads();
-  for (int i = warp; i < Mech::NS; i += kWarps) {
+  for (int i = warp; i < Mech::NS; i += kRateWarps) {
     const int begin = T::f_ptr[i], end = T::f_ptr[i + 1];
-    double v = begin < end ? -0.0 : 0.0;  // c * t + (-0) is c * t
-    for (int t = begin; t < end; ++t) v = fma(T::f_coef[t], q[T::f_term[t] * 32 + lane], v);
+    double v = begin < end ? first_term(T::f_coef[begin], q[T::f_term[begin] * 32 + lane]) : 0.0;
+    for (int t = begin + 1; t < end; ++t) v = fma(T::f_coef[t], q[T::f_term[t] * 32 + lane], v);
     if (cell < n) out[cell + n * i] = v;
   }
 }
 
-// Column blockIdx.y of the Jacobian of 32 cells.
+// Column blockIdx.y of the Jacobian of 32 * kCells cells, kCells per lane.
+template <int kCells>
 __global__ void __launch_bounds__(kWarps * 32) eval_jacobian_kernel(size_t n, const double* __restrict__ conc,
                                                                    const double* __restrict__ ktab,
                                                                    double* __restrict__ out) {
-  extern __shared__ double d[];  // [partial of the column][lane]
+  extern __shared__ double d[];  // [partial of the column][cell]
+  constexpr int kRow = 32 * kCells;
   const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  const size_t cell = blockIdx.x * (size_t)32 + lane;
-  const size_t c = cell < n ? cell : n - 1;
+  const size_t cell = blockIdx.x * (size_t)kRow + lane;
   const int col = blockIdx.y;
   const int first = T::p_ptr[col], count = T::p_ptr[col + 1] - first;
-  for (int p = warp; p < count; p += kWarps)
-    d[p * 32 + lane] = product(__ldg(ktab + c + n * T::p_rate[first + p]), T::p_product[first + p], conc, c, n);
+  for (int p = warp; p < count; p += kWarps) {
+    const double* k = ktab + n * T::p_rate[first + p];
+    const unsigned code = T::p_product[first + p];
+#pragma unroll
+    for (int i = 0; i < kCells; ++i) {
+      const size_t c = cell + 32 * i < n ? cell + 32 * i : n - 1;
+      d[p * kRow + 32 * i + lane] = product(__ldg(k + c), code, conc, c, n);
+    }
+  }
   __syncthreads();
   double* column = out + n * (size_t)Mech::NS * col + cell;
+  const unsigned* entries = T::j_ptr + Mech::NS * col;
   for (int row = warp; row < Mech::NS; row += kWarps) {
-    const unsigned entry = T::j_ptr[row + Mech::NS * col];
-    double v = 0.0;
+    const unsigned entry = entries[row];
+    double v[kCells];
+#pragma unroll
+    for (int i = 0; i < kCells; ++i) v[i] = 0.0;
     if (entry & 2u) {  // -W with 1/(gamma h) = 0, which the diagonal's sum starts from
-      const int begin = entry >> 2, end = T::j_ptr[row + Mech::NS * col + 1] >> 2;
-      double w = (entry & 1u) || begin == end ? 0.0 : -0.0;
-      for (int t = begin; t < end; ++t) w = fma(T::j_coef[t], d[T::j_term[t] * 32 + lane], w);
-      v = -w;
+      const int end = entries[row + 1] >> 2;
+      int t = entry >> 2;
+      if (!(entry & 1u) && t < end) {
+#pragma unroll
+        for (int i = 0; i < kCells; ++i) v[i] = first_term(T::j_coef[t], d[T::j_term[t] * kRow + 32 * i + lane]);
+        ++t;
+      }
+      for (; t < end; ++t) {
+#pragma unroll
+        for (int i = 0; i < kCells; ++i) v[i] = fma(T::j_coef[t], d[T::j_term[t] * kRow + 32 * i + lane], v[i]);
+      }
+#pragma unroll
+      for (int i = 0; i < kCells; ++i) v[i] = -v[i];
     }
-    if (cell < n) column[n * row] = v;
+#pragma unroll
+    for (int i = 0; i < kCells; ++i)
+      if (cell + 32 * i < n) column[n * row + 32 * i] = v[i];
   }
+}
+
+template <int kCells>
+int launch_jacobian(size_t n, const double* conc, const double* ktab, double* out, cudaStream_t stream) {
+  constexpr size_t kSmem = (size_t)(T::MAX_PARTIALS > 0 ? T::MAX_PARTIALS : 1) * 32 * kCells * sizeof(double);
+  if (kSmem > kDefaultSmem && cudaFuncSetAttribute(eval_jacobian_kernel<kCells>,
+                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem) != cudaSuccess)
+    return MKPP_ERROR_DEVICE;
+  eval_jacobian_kernel<kCells><<<dim3(launch_grid(n, 32 * kCells), Mech::NS), kWarps * 32, kSmem, stream>>>(n, conc, ktab,
+                                                                                                           out);
+  return cudaGetLastError() == cudaSuccess ? MKPP_SUCCESS : MKPP_ERROR_DEVICE;
 }
 
 // Columns of the dense Jacobian that belong to fixed species (through the
@@ -155,7 +195,7 @@ int launch_eval_rates(size_t n, const double* conc, const double* ktab, double* 
       cudaFuncSetAttribute(eval_rates_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRatesSmem) !=
           cudaSuccess)
     return MKPP_ERROR_DEVICE;
-  eval_rates_kernel<<<launch_grid(n, 32), kWarps * 32, kRatesSmem, stream>>>(n, conc, ktab, out);
+  eval_rates_kernel<<<launch_grid(n, 32), kRateWarps * 32, kRatesSmem, stream>>>(n, conc, ktab, out);
   return cudaGetLastError() == cudaSuccess ? MKPP_SUCCESS : MKPP_ERROR_DEVICE;
 }
 
@@ -164,12 +204,12 @@ int launch_eval_jacobian(size_t n, const double* conc, const double* ktab, doubl
     eval_cell_jacobian_kernel<Mech><<<launch_grid(n, 128), 128, 0, stream>>>(n, conc, ktab, out);
     return cudaGetLastError() == cudaSuccess ? MKPP_SUCCESS : MKPP_ERROR_DEVICE;
   }
-  if (kJacSmem > kDefaultSmem &&
-      cudaFuncSetAttribute(eval_jacobian_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kJacSmem) !=
-          cudaSuccess)
-    return MKPP_ERROR_DEVICE;
-  eval_jacobian_kernel<<<dim3(launch_grid(n, 32), Mech::NS), kWarps * 32, kJacSmem, stream>>>(n, conc, ktab, out);
-  return cudaGetLastError() == cudaSuccess ? MKPP_SUCCESS : MKPP_ERROR_DEVICE;
+  // Two cells per lane halve the table reads of an output (SAPRC99, 20000
+  // cells: 279 -> 243 us), but need twice the shared memory (TS1, 30 KB for a
+  // column of one cell a lane: 107 -> 137 us for 1001 cells) and enough blocks
+  // (100 SAPRC99 cells: 17 us, 23 with two).
+  if (T::MAX_PARTIALS <= 96 && n >= 2048) return launch_jacobian<2>(n, conc, ktab, out, stream);
+  return launch_jacobian<1>(n, conc, ktab, out, stream);
 }
 
 int launch_fixed_columns(size_t n, const double* conc, const double* temp, const double* rho, const double* rh,

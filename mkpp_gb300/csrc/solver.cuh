@@ -102,9 +102,9 @@ struct ZeroRow {
 
 // A thread has one cell and one part of the reactions (blockIdx.y), so that a
 // small call spreads over the SMs: FP64 transcendentals, whose instructions a
-// warp issues one per 64 cycles, bound it (SAPRC99, 100 cells: 263 us with all
-// 211 reactions on a thread).  With the parts the evaluation of 1001 TS1 cells
-// went from 0.94 to 0.32 ms, of 20000 SAPRC99 cells from 0.83 to 0.66 ms.
+// warp issues one per 64 cycles, bound it.  SAPRC99: 100 cells 42 us, 263 with all
+// 211 reactions on a thread, 20000 cells 290 us, 445; TS1, 1001 cells: 65 us, 650
+// before and 137 with parts of eight reactions whatever their functions.
 template <class Mech>
 __global__ void __launch_bounds__(128) rate_constant_kernel(RateArgs a) {
   const size_t n = (size_t)a.ncells;
@@ -527,7 +527,7 @@ __device__ __forceinline__ void coop_integrate_cell(const LaunchArgs& a, double*
       }
       const double h = ctl.next_h();
       int st = 0;
-      const double err = Mech::attempt_coop(S, h, st, lane, WarpProgram());
+      const double err = Mech::attempt_coop(S, h, st, lane, WarpProgram<Mech::PIVOT_EVERY>());
       zero_pivot |= st != 0;
       if (ctl.update<Mech>(err)) {
         for (int i = lane; i < Mech::NV; i += 32) S[Mech::Y + i] += S[Mech::DY + i];

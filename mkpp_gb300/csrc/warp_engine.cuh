@@ -11,7 +11,8 @@ constexpr int kProgramAhead = 8;
 
 // One warp runs `steps` steps (a multiple of kProgramAhead, the last one idle)
 // of 32 words, a lane per word, two steps' words of a lane side by side, on
-// one store that the warp shares.
+// one store that the warp shares; reciprocals only in the last of kPivotEvery
+// steps.
 //
 // Bound by latency: a GB300 warp issues one FP64 instruction per 64 cycles,
 // whatever its active lanes, and any other instruction gets the result ~40
@@ -20,6 +21,7 @@ constexpr int kProgramAhead = 8;
 // up to four warps on an SM and 165 with eight (the FP64 pipe's bound there is
 // 152), against 172 and 204 with a vote for pivots in every step, operand
 // loads under branches and the words of a step each waited for alone.
+template <int kPivotEvery>
 struct WarpProgram {
   // Returns false if a reciprocal of this lane met a zero.
   __device__ __forceinline__ bool operator()(double* S, const unsigned long long* __restrict__ prog, int steps,
@@ -56,7 +58,7 @@ struct WarpProgram {
         const double b = p.prev_b() ? prev : B;
         const double c = p.prev_c() ? prev : C;
         double v = fma(A, b, c);
-        if constexpr (decltype(pivots)::value) {
+        if (decltype(pivots)::value && j % kPivotEvery == kPivotEvery - 1) {
           if (__any_sync(0xffffffffu, p.reciprocal())) {
             ok = ok && !(p.reciprocal() && is_zero(b));
             const double r = divide(1.0, p.reciprocal() ? b : 1.0);

@@ -89,8 +89,22 @@ def _sum_expr(init: str | None, terms: list[tuple[float, str]]) -> str:
 
 
 ILP_GROUP = 8
-# Reactions per block of the rate-constant kernel.
-RATE_PART = 8
+# Work of one part of the rate constants, in exponentials: a power takes about
+# 150 FP64 instructions, three times an exponential, and a warp issues one per
+# 64 cycles, so a part of eight Troe reactions took 113 us however few the cells.
+RATE_PART = 4.0
+
+
+def _rate_parts(reactions):
+    parts, work = [[]], 0.0
+    for r in reactions:
+        own = 0.2 + 3.0 * r.k.count("pow(") + r.k.count("exp(") + r.k.count("log(")
+        if parts[-1] and work + own > RATE_PART:
+            parts.append([])
+            work = 0.0
+        parts[-1].append(r)
+        work += own
+    return parts
 # Slot count above which the solver keeps a cell's working set in the global
 # tile rather than registers (kRegisterSlots in csrc/solver.cuh).
 REGISTER_SLOTS = 96
@@ -138,6 +152,13 @@ def _c_u64_array(c, name, values):
     c("};")
 
 
+def _c_program(c, count, name, ops):
+    """A program of one thread: its words and their number."""
+    words = warp_schedule.encode(ops, warp_schedule.sequential(ops), lanes=1)
+    c(f"constexpr int {count} = {len(words)};")
+    _c_u64_array(c, name, words)
+
+
 def _shifted(ops, first, by):
     """The operations with the slots from `first` on moved down."""
     return [(op[0], *(x - by if x >= first else x for x in op[1:5]), op[5]) for op in ops]
@@ -157,14 +178,21 @@ def _coop_build(plan, nv, stages, A, C, NewF, K0, Y, FS, DY, nslots, table=False
     npart = sum(len(r.reactants) for r in plan.reactions)
     Q = nslots                      # rates q_r (then q_i of the error norm)
     D = nslots + nq                 # Jacobian partial derivatives
-    CB = D + npart                  # constants: -0, +0, 1, 1/(gamma h), c_ij/h, literals
+    # The partials live between the state and W, when the LU's fill-in slots
+    # have no value yet: they sit there as far as those go, which makes TS1's
+    # store small enough for four warps per SM.
+    fill = warp_schedule.lu_zero_slots(plan)
+    part_slot = [fill[p] if p < len(fill) else D + p - len(fill) for p in range(npart)]
+    extra_parts = max(0, npart - len(fill))
+    # (The table-driven per-thread store keeps its size.)
+    CB = D + (npart if table else extra_parts)  # constants: -0, +0, 1, 1/(gamma h), c_ij/h, literals
     # The table-driven adjoint's slots sit before the constants.  The
     # cooperative kernel's store does without them: its slots from the
     # constants on are `shift` lower.
     adj = _adjoint_layout(CB, nv, nr, stages) if table else None
     shift = 0
     if table:
-        shift = adj["end"] - CB
+        shift = adj["end"] - D - extra_parts
         CB = adj["end"]
     ZN, ZP, ONE, IG = CB, CB + 1, CB + 2, CB + 3
     cterm_slot = {}
@@ -221,9 +249,9 @@ def _coop_build(plan, nv, stages, A, C, NewF, K0, Y, FS, DY, nslots, table=False
                     else:
                         fac += [Y + v2l[s2]] * pw2
                 if not fac:
-                    P.copy(D + p, Mech_KT + r.index)
+                    P.copy(part_slot[p], Mech_KT + r.index)
                 for n_, f in enumerate(fac):
-                    P.mul(D + p, (Mech_KT + r.index) if n_ == 0 else D + p, f)
+                    P.mul(part_slot[p], (Mech_KT + r.index) if n_ == 0 else part_slot[p], f)
                 pidx[(r.index, s_)] = p
                 p += 1
         wterms = {loc: [] for loc in plan.w_slots}
@@ -238,12 +266,12 @@ def _coop_build(plan, nv, stages, A, C, NewF, K0, Y, FS, DY, nslots, table=False
                 if not terms:
                     P.copy(out, IG)
                 for n_, (coef, pi) in enumerate(terms):
-                    P.acc_term(out, False, float(coef), D + pi, acc=IG if n_ == 0 else None)
+                    P.acc_term(out, False, float(coef), part_slot[pi], acc=IG if n_ == 0 else None)
             else:
                 if not terms:
                     P.zero(out)
                 for n_, (coef, pi) in enumerate(terms):
-                    P.acc_term(out, n_ == 0, float(coef), D + pi)
+                    P.acc_term(out, n_ == 0, float(coef), part_slot[pi])
         for sl in warp_schedule.lu_zero_slots(plan):
             P.zero(sl)
 
@@ -312,7 +340,8 @@ def _coop_build(plan, nv, stages, A, C, NewF, K0, Y, FS, DY, nslots, table=False
     nconst = len(const_vals)
     seq_ops = [op for ops in progs for op in ops] if table else None
     return {"progs": progs, "warp": warp, "shift": shift, "sched": sched, "seq_ops": seq_ops,
-            "npart": npart, "nq": nq, "Q": Q, "D": D, "CB": CB, "nconst": nconst, "const_vals": const_vals, "literals": literals, "cterm_slot": cterm_slot,
+            "npart": npart, "nq": nq, "Q": Q, "D": D, "CB": CB, "nconst": nconst,
+            "const_vals": const_vals, "literals": literals, "cterm_slot": cterm_slot,
             "KT": Mech_KT, "total": CB + nconst, "adj": adj, "adj_ops": adj_ops, "eval_ops": eval_ops,
             "A": A, "NewF": NewF}
 
@@ -741,9 +770,8 @@ def _emit_tlm(c, t, tlm, C):
     """Constants, tables (into the coop namespace text t) and tlm_step."""
     L = tlm["L"]
     ops = tlm["ops"]
-    t(f"constexpr int TLM_OPS = {len(ops)};")
     t(f"static __device__ const double tlm_const_val[{tlm['nconst']}] = {{{', '.join(tlm['const_vals'])}}};")
-    _c_u64_array(t, "tlm_prog", warp_schedule.encode(ops, [[i] for i in range(len(ops))], lanes=1))
+    _c_program(t, "TLM_OPS", "tlm_prog", ops)
     c("")
     c("  // ---- tangent of one accepted step (forward sensitivities) ----")
     c(f"  static constexpr int DYT = {L['DYT']};     // dy in, dy_new out (NV)")
@@ -761,7 +789,7 @@ def _emit_tlm(c, t, tlm, C):
     for (st, j), slot in tlm["cterm"].items():
         cv = C[(st - 1) * (st - 2) // 2 + j - 1]
         c(f"    S[{slot}] = mkpp::divide({_lit(cv)}, h);    // c{st}{j} / h")
-    c("    mkpp::run_program(S, coop::tlm_prog, coop::TLM_OPS);")
+    c("    mkpp::run_program<false>(S, coop::tlm_prog, coop::TLM_OPS);")
     c("  }")
 
 
@@ -784,7 +812,7 @@ def _emit_table_adjoint(c, coop):
     c("  __device__ __forceinline__ static void adjoint_step(SA& S, const KA& k, double h) {")
     c("    (void)k;")
     c("    (void)h;")
-    c("    mkpp::run_program(S, coop::adj_prog, coop::ADJ_OPS);")
+    c("    mkpp::run_program<false>(S, coop::adj_prog, coop::ADJ_OPS);")
     c("  }")
     c("")
     c("  // ---- tendencies and Jacobian (table-driven evaluation entries) ----")
@@ -796,7 +824,7 @@ def _emit_table_adjoint(c, coop):
     c("    for (int r = 0; r < NR; ++r) S[KT + r] = k(r);")
     c("    for (int i = 0; i < NCONST; ++i) S[CB + i] = coop::const_val[i];")
     c("    S[CB + 3] = 0.0;  // 1/(gamma h)")
-    c("    mkpp::run_program(S, coop::eval_prog, coop::EVAL_OPS);")
+    c("    mkpp::run_program<false>(S, coop::eval_prog, coop::EVAL_OPS);")
     c("  }")
 
 
@@ -816,7 +844,7 @@ def _emit_table_attempt_head(c, coop, C):
     for (st, j), slot in coop["cterm_slot"].items():
         cv = C[(st - 1) * (st - 2) // 2 + j - 1]
         c(f"    S[{slot}] = mkpp::divide({_lit(cv)}, h);    // c{st}{j} / h")
-    c("    if (!mkpp::run_program(S, coop::attempt_prog, coop::ATTEMPT_OPS)) status |= 1;")
+    c("    if (!mkpp::run_program<true>(S, coop::attempt_prog, coop::ATTEMPT_OPS)) status |= 1;")
 
 
 def _emit_coop(c, plan, coop, nv, ns, stages, C, M, E, K0, Y, FS, DY):
@@ -831,10 +859,11 @@ def _emit_coop(c, plan, coop, nv, ns, stages, C, M, E, K0, Y, FS, DY):
     c("  // ---- warp-cooperative attempt (static warp schedules) ----")
     c(f"  static constexpr int NPART = {npart};")
     c(f"  static constexpr int Q = {Q};            // rates q_r, then q_i of the error norm")
-    c(f"  static constexpr int D = {D};     // partial derivatives")
+    c(f"  static constexpr int D = {D};     // partial derivatives beyond the LU's fill-in slots")
     c(f"  static constexpr int CB = {CB};        // constants")
     c(f"  static constexpr int NCONST = {nconst};")
     c(f"  static constexpr int COOP_SLOTS = CB + NCONST;")
+    c(f"  static constexpr int PIVOT_EVERY = {warp_schedule.pivot_every(progs[0])};  // steps that may hold reciprocals")
     c(f"  static constexpr int WCB = {CB - coop['shift']};       // constants in the store of a warp")
     c(f"  static constexpr int WARP_SLOTS = WCB + NCONST;")
     t = _Code()
@@ -856,16 +885,13 @@ def _emit_coop(c, plan, coop, nv, ns, stages, C, M, E, K0, Y, FS, DY):
     _c_u64_array(t, "sched", words)
     if coop["seq_ops"] is not None:
         ops = coop["seq_ops"]
-        t(f"constexpr int ATTEMPT_OPS = {len(ops)};")
-        _c_u64_array(t, "attempt_prog", warp_schedule.encode(ops, [[i] for i in range(len(ops))], lanes=1))
+        _c_program(t, "ATTEMPT_OPS", "attempt_prog", ops)
     if coop["adj_ops"] is not None:
         ops = coop["adj_ops"]
-        t(f"constexpr int ADJ_OPS = {len(ops)};")
-        _c_u64_array(t, "adj_prog", warp_schedule.encode(ops, [[i] for i in range(len(ops))], lanes=1))
+        _c_program(t, "ADJ_OPS", "adj_prog", ops)
     if coop["eval_ops"] is not None:
         ops = coop["eval_ops"]
-        t(f"constexpr int EVAL_OPS = {len(ops)};")
-        _c_u64_array(t, "eval_prog", warp_schedule.encode(ops, [[i] for i in range(len(ops))], lanes=1))
+        _c_program(t, "EVAL_OPS", "eval_prog", ops)
     tlm = _tlm_build(plan, nv, stages, coop["A"], C, M, coop["NewF"], K0, Y, Mech_KT, coop["total"])
     tlm_code = _Code()
     _emit_tlm(tlm_code, t, tlm, C)
@@ -1316,7 +1342,7 @@ def emit_mechanism(plan: ReducedPlan, table: bool | None = None) -> str:
     c("  // FIX(s) the concentration of fixed species s, T/RHO the cell's")
     c("  // temperature and air density.  In parts of a few reactions, which the")
     c("  // rate kernel gives to different blocks.")
-    parts = [plan.reactions[i:i + RATE_PART] for i in range(0, nr, RATE_PART)]
+    parts = _rate_parts(plan.reactions)
     c(f"  static constexpr int RATE_PARTS = {len(parts)};")
     c("  template <class PA, class FA, class KO>")
     c("  __device__ __forceinline__ static void rate_constants_part(int part, const PA& P, const FA& FIX, double T,")

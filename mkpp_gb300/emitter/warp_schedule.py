@@ -206,10 +206,19 @@ def schedule(ops, lanes: int = LANES) -> list[list[int]]:
 LOAD = 2              # steps from an operation to a reader through its slot
 
 
+def pivot_every(ops) -> int:
+    """Steps from one that may hold reciprocals to the next.  Each of them
+    costs the device loop a vote, and one with a reciprocal several steps, so a
+    long program gathers them (SAPRC99: 37 steps instead of 56, TS1 104 instead
+    of 163, at the same length); a short one would wait for them."""
+    return AHEAD if len(ops) >= 5000 else 1
+
+
 def pipeline(ops, lanes: int = LANES) -> list[list[int | None]]:
     """Steps of `lanes` entries (an operation or None) for the device loop.
     Priority: longest remaining path, a sum's next term one step after, any
     other reader LOAD steps."""
+    every = pivot_every(ops)
     n = len(ops)
     raw: list[list[int]] = []
     raw_succ: list[list[int]] = [[] for _ in range(n)]
@@ -237,7 +246,7 @@ def pipeline(ops, lanes: int = LANES) -> list[list[int | None]]:
     tail = [1] * n
     for i in range(n - 1, -1, -1):
         for t in raw_succ[i]:
-            lag = 1 if ops[t][0] == RCP or ops[t][4] == ops[i][1] else LOAD
+            lag = (every + 1) // 2 if ops[t][0] == RCP else 1 if ops[t][4] == ops[i][1] else LOAD
             tail[i] = max(tail[i], lag + tail[t])
         for t, lag in other_succ[i]:
             tail[i] = max(tail[i], lag + tail[t])
@@ -273,11 +282,20 @@ def pipeline(ops, lanes: int = LANES) -> list[list[int | None]]:
             if left[t] == 0:
                 release(t)
 
+    pivots: list[tuple[int, int]] = []
+
     while done < n:
         for i in from_slots.pop(s, ()):
             if step[i] < 0:
                 heapq.heappush(ready, (-tail[i], i))
         follow = sorted((-tail[i], i, j) for i, j in forwarded.pop(s, ()))
+        # Reciprocals wait for a step that has the code for them.
+        pivot_step = s % every == every - 1
+        if pivot_step:
+            while pivots:
+                heapq.heappush(ready, heapq.heappop(pivots))
+        else:
+            follow = [x for x in follow if ops[x[1]][0] != RCP]
         used: set[int] = set()
         anywhere = []
         f = count = 0
@@ -290,8 +308,12 @@ def pipeline(ops, lanes: int = LANES) -> list[list[int | None]]:
                 lane[i] = lane[j]
                 used.add(lane[i])
             else:
-                i = heapq.heappop(ready)[1]
+                top = heapq.heappop(ready)
+                i = top[1]
                 if step[i] >= 0:
+                    continue
+                if ops[i][0] == RCP and not pivot_step:
+                    pivots.append(top)
                     continue
                 anywhere.append(i)
             place(i)
@@ -305,6 +327,17 @@ def pipeline(ops, lanes: int = LANES) -> list[list[int | None]]:
     for i in range(n):
         rows[step[i]][lane[i]] = i
     return rows
+
+
+def sequential(ops) -> list[list[int]]:
+    """One operation per step, for a single thread; an idle step before the
+    square of the result just made (one factor can be forwarded)."""
+    steps: list[list[int]] = []
+    for i, op in enumerate(ops):
+        if i and op[0] == FMA and op[2] == op[3] == ops[i - 1][1]:
+            steps.append([])
+        steps.append([i])
+    return steps
 
 
 def encode(ops, steps, lanes: int = LANES) -> list[int]:
@@ -335,7 +368,7 @@ def encode(ops, steps, lanes: int = LANES) -> list[int]:
         from_slot = ([a] if kind == FMA else []) + ([] if x_b else [b]) + ([c] if kind == FMA and not x_c else [])
         for x in from_slot:
             if x in last:
-                assert lanes == 1 or where[last[x]][0] <= where[i][0] - LOAD
+                assert where[last[x]][0] <= where[i][0] - LOAD
                 stored[last[x]] = True
         fields[i] = (a, PREV if x_b else b, PREV if x_c else c)
         last[out] = i

@@ -63,12 +63,17 @@ def test_evaluation_does_not_depend_on_the_batch(libs, mech):
     from mkpp_gb300.api import DeviceSolver
 
     s = DeviceSolver(mech)
-    w = workloads.make(mech, 97, seed=6)
+    total = 2081                    # two cells per lane of the Jacobian's blocks, the last ones alone
+    w = workloads.make(mech, total, seed=6)
     d = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()  # noqa: E731
     conc = d(w.conc)
     k, _ = s.rate_constants(conc, d(w.temp), d(w.rho), d(w.rh), None, d(w.param))
     f, j = s.evaluate_rates(conc, k), s.evaluate_jacobian(conc, k)
     for n in (1, 31, 32, 33, 64, 65):
-        sub, ks = conc[:, 97 - n:].contiguous(), k[:, 97 - n:].contiguous()
-        assert torch.equal(s.evaluate_rates(sub, ks), f[:, 97 - n:])
-        assert torch.equal(s.evaluate_jacobian(sub, ks), j[:, :, 97 - n:])
+        at = total - n
+        sub, ks = conc[:, at:].contiguous(), k[:, at:].contiguous()
+        cut = lambda a: d(a[..., at:])  # noqa: E731
+        again, flagged = s.rate_constants(sub, cut(w.temp), cut(w.rho), cut(w.rh), None, cut(w.param))
+        assert torch.equal(again, ks) and not flagged.any()
+        assert torch.equal(s.evaluate_rates(sub, ks), f[:, at:])
+        assert torch.equal(s.evaluate_jacobian(sub, ks), j[:, :, at:])
