@@ -119,6 +119,40 @@ __device__ __forceinline__ double divide(double a, double b) {
 #endif
 }
 
+// a < b, and the smaller, of numbers that are zero or positive (not NaN), by
+// their bit patterns.
+__device__ __forceinline__ bool below(double a, double b) {
+  return __double_as_longlong(a) < __double_as_longlong(b);
+}
+__device__ __forceinline__ double least(double a, double b) { return below(b, a) ? b : a; }
+// fmax(x, floor) for a positive floor and x zero, positive or NaN.
+__device__ __forceinline__ double at_least(double x, double floor) {
+  const long long bits = __double_as_longlong(x);
+  return bits > (0x7ffll << 52) || bits < __double_as_longlong(floor) ? floor : x;
+}
+
+// A number of the rate expressions whose divisions are divide(): nearly every
+// rate constant divides by the temperature.
+struct Num {
+  double v;
+  __device__ __forceinline__ Num(double x) : v(x) {}
+  __device__ __forceinline__ friend Num operator+(Num a, Num b) { return a.v + b.v; }
+  __device__ __forceinline__ friend Num operator-(Num a, Num b) { return a.v - b.v; }
+  __device__ __forceinline__ friend Num operator*(Num a, Num b) { return a.v * b.v; }
+  __device__ __forceinline__ friend Num operator/(Num a, Num b) { return divide(a.v, b.v); }
+  __device__ __forceinline__ friend Num operator-(Num a) { return -a.v; }
+  __device__ __forceinline__ friend Num exp(Num a) { return ::exp(a.v); }
+  __device__ __forceinline__ friend Num log(Num a) { return ::log(a.v); }
+  __device__ __forceinline__ friend Num sqrt(Num a) { return ::sqrt(a.v); }
+  __device__ __forceinline__ friend Num fabs(Num a) { return ::fabs(a.v); }
+  __device__ __forceinline__ friend Num pow(Num a, int b) { return ::pow(a.v, b); }
+  __device__ __forceinline__ friend Num pow(Num a, double b) { return ::pow(a.v, b); }
+  __device__ __forceinline__ friend Num pow(Num a, Num b) { return ::pow(a.v, b.v); }
+  __device__ __forceinline__ friend Num pow(double a, Num b) { return ::pow(a, b.v); }
+};
+__device__ __forceinline__ double value(double x) { return x; }
+__device__ __forceinline__ double value(Num x) { return x.v; }
+
 // fmax(fabs(x), fabs(y)) by the bit patterns, off the FP64 pipe.
 __device__ __forceinline__ double max_abs(double x, double y) {
   const unsigned long long mask = ~(1ull << 63), inf = 0x7ffull << 52;

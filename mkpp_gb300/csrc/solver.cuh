@@ -102,9 +102,10 @@ struct ZeroRow {
 
 // A thread has one cell and one part of the reactions (blockIdx.y), so that a
 // small call spreads over the SMs: FP64 transcendentals, whose instructions a
-// warp issues one per 64 cycles, bound it.  SAPRC99: 100 cells 42 us, 263 with all
-// 211 reactions on a thread, 20000 cells 290 us, 445; TS1, 1001 cells: 65 us, 650
-// before and 137 with parts of eight reactions whatever their functions.
+// warp issues one per 64 cycles, bound it.  SAPRC99: 100 cells 47 us, 263 with all
+// 211 reactions on a thread; 20000 cells 263 us, 290 with the hardware's divisions
+// (Num), 445; TS1, 1001 cells: 63 us, 650 before and 137 with parts of eight
+// reactions whatever their functions.
 template <class Mech>
 __global__ void __launch_bounds__(128) rate_constant_kernel(RateArgs a) {
   const size_t n = (size_t)a.ncells;
@@ -119,10 +120,10 @@ __global__ void __launch_bounds__(128) rate_constant_kernel(RateArgs a) {
   CheckedRowOut k{a.ktab + c, n, true};
   if (a.param) {
     CellRow P{a.param + c, n};
-    Mech::rate_constants_part(part, P, fix, T, RHO, RH, CLW, k);
+    Mech::rate_constants_part(part, P, fix, Num(T), Num(RHO), Num(RH), Num(CLW), k);
   } else {
     ZeroRow P;
-    Mech::rate_constants_part(part, P, fix, T, RHO, RH, CLW, k);
+    Mech::rate_constants_part(part, P, fix, Num(T), Num(RHO), Num(RH), Num(CLW), k);
   }
   if (a.status) {  // all CELL_SUCCESS before the launch
     bool ok = k.ok && finite(T) && finite(RHO);
@@ -180,6 +181,9 @@ __device__ __forceinline__ RegStore<N> make_store(double*, RegStore<N>*, unsigne
 // ---------------------------------------------------------------------------
 // Per-cell controller state and one controller step.
 // ---------------------------------------------------------------------------
+// The times, step sizes and error norms it compares are positive numbers
+// (Mech::attempt's norm is at least 1e-10, whatever the stages hold), so it
+// compares their bit patterns, off the FP64 pipe.
 struct Controller {
   double t, dt, dt_total, h_min;
   double want;       // the step size chosen before the end-of-call cut
@@ -198,12 +202,13 @@ struct Controller {
     reject_last = reject_more = cut = false;
     attempts = 0;
   }
-  __device__ __forceinline__ bool running() const { return t < dt_total; }
+  __device__ __forceinline__ bool running() const { return below(t, dt_total); }
   // Step size of the next attempt (integrate.j2:85: dt = min(dt, dt_total - t)).
   __device__ __forceinline__ double next_h() {
     want = dt;
-    cut = dt_total - t < dt;
-    dt = fmin(dt, dt_total - t);
+    const double rest = dt_total - t;
+    cut = below(rest, dt);
+    dt = cut ? rest : dt;
     return dt;
   }
   // Step size carried into the next call once this one has ended: the
@@ -215,10 +220,11 @@ struct Controller {
   __device__ __forceinline__ bool update(double err) {
     const double factor = Mech::growth(err);
     ++attempts;
-    if (err <= 1.0) {
+    if (!below(1.0, err)) {
       t += dt;
-      double next_dt = fmax(h_min, fmin(dt * factor, dt_total));
-      if (reject_last) next_dt = fmin(next_dt, dt);
+      double next_dt = least(dt * factor, dt_total);
+      next_dt = below(h_min, next_dt) ? next_dt : h_min;
+      if (reject_last) next_dt = least(next_dt, dt);
       reject_last = false;
       reject_more = false;
       dt = next_dt;

@@ -960,7 +960,7 @@ def _emit_coop(c, plan, coop, nv, ns, stages, C, M, E, K0, Y, FS, DY):
     c("    double err_sq = 0.0;")
     c("    #pragma unroll 8")
     c("    for (int i = 0; i < NV; ++i) err_sq = fma(S[Q + i], S[Q + i], err_sq);")
-    c(f"    return fmax(sqrt(mkpp::divide(err_sq, {ns}.0)), 1.0e-10);")
+    c(f"    return mkpp::at_least(sqrt(mkpp::divide(err_sq, {ns}.0)), 1.0e-10);")
     c("  }")
     for line in tlm_code.lines:
         c(line)
@@ -1344,15 +1344,16 @@ def emit_mechanism(plan: ReducedPlan, table: bool | None = None) -> str:
     c("  // rate kernel gives to different blocks.")
     parts = _rate_parts(plan.reactions)
     c(f"  static constexpr int RATE_PARTS = {len(parts)};")
-    c("  template <class PA, class FA, class KO>")
-    c("  __device__ __forceinline__ static void rate_constants_part(int part, const PA& P, const FA& FIX, double T,")
-    c("                                                           double RHO, double RH, double CLW, KO& k) {")
+    c("  // V is double, or mkpp::Num, whose divisions take the integer pipes.")
+    c("  template <class PA, class FA, class KO, class V>")
+    c("  __device__ __forceinline__ static void rate_constants_part(int part, const PA& P, const FA& FIX, V T, V RHO,")
+    c("                                                           V RH, V CLW, KO& k) {")
     c("    (void)T; (void)RHO; (void)RH; (void)CLW; (void)P; (void)FIX;")
     c("    switch (part) {")
     for i, part in enumerate(parts):
         c(f"      case {i}:")
         for r in part:
-            c(f"        k.set({r.index}, {_k_text(r.k)});")
+            c(f"        k.set({r.index}, mkpp::value({_k_text(r.k)}));")
         c("        break;")
     c("    }")
     c("  }")
@@ -1642,7 +1643,7 @@ def emit_mechanism(plan: ReducedPlan, table: bool | None = None) -> str:
     c(f"      const double q = {div.format('(' + lin(eterms) + ')', 'sc')};")
     c("      err_sq = fma(q, q, err_sq);")
     c("    }")
-    c(f"    return fmax(sqrt(mkpp::divide(err_sq, {ns}.0)), 1.0e-10);")
+    c(f"    return mkpp::at_least(sqrt(mkpp::divide(err_sq, {ns}.0)), 1.0e-10);")
     c("  }")
     c("")
     c("  // Step-size factor from the error norm (integrate.j2:324-333).")
@@ -1653,7 +1654,7 @@ def emit_mechanism(plan: ReducedPlan, table: bool | None = None) -> str:
         c("    const double fac = mkpp::divide(0.9, cbrt(err));")
     else:
         c(f"    const double fac = 0.9 * pow(err, -{_lit(1.0 / elo)});")
-    c("    return fmax(0.2, fmin(fac, 6.0));")
+    c("    return mkpp::at_least(mkpp::least(fac, 6.0), 0.2);")
     c("  }")
     _emit_coop(c, plan, coop, nv, ns, stages, C, M, E, K0, Y, FS, DY)
     if table:
