@@ -116,8 +116,8 @@ int device_fail(mkpp_handle_s* h, cudaError_t err, const char* what) {
 //                    cell after defer_after * S attempts in all.  A
 //                    cooperative SAPRC99 attempt takes ~0.19 ms against
 //                    ~1 ms on one lane, but the cooperative kernel has about
-//                    a fifth of the lanes' throughput, so only the tail
-//                    should park.  The default, 3000, parks ~7% of the cells
+//                    a quarter of the full lanes' throughput, so only the
+//                    tail should park.  The default, 3000, parks ~7% of the cells
 //                    in the stiff first host step of the SAPRC99 workload,
 //                    ~0.15% (its slowest cells) in the later ones, and none
 //                    in a 24-step window (whose slowest cell needs ~22000).
@@ -146,18 +146,17 @@ struct Tuning {
   int split_cells = 0;
   int split_sms = 0;
   // Calls of at most this many cells run on the cooperative kernel alone
-  // (coop_alone).  A lane needs 1.0 ms for a SAPRC99 attempt
-  // and 1.9 ms with every SM full, a warp 0.19 ms; with eight warps per SM the
-  // warps reach 5.2 M attempts/s against the lanes' 2.9 M in one host step of
-  // 32768 cells (206 against 371 ms; 2500 cells: 34 against 163 ms), and the
-  // lanes' 6.2 M in four host steps of 65536.  A table-driven mechanism (TS1)
-  // is always faster there: 79 against 293 ms for 4096 cells.  A mechanism
-  // with few operations per attempt spends them on the parts that every lane
-  // of the warp repeats: saprc99_mini wins up to 8192 cells (2500 cells: 1.38
-  // against 3.14 ms; 32768: 8.8 against 7.2 ms), one whose lanes keep their
-  // store in registers a few hundred (small_strato: 72 cells 1.8 against 3.1
-  // ms, 4096 cells 6.1 against 3.5; Chapman: 0.50 against 0.60 ms, 2.1 against
-  // 0.67).
+  // (coop_alone).  A lane needs 1.0 ms for a SAPRC99 attempt and 1.9 ms with
+  // every SM full, a warp 0.17-0.19 ms; with eight warps per SM the warps reach
+  // 5.5 M attempts/s.  One host step: 2500 cells 34 against 163 ms, 8000 cells 55
+  // against 59, 14000 equal, 20000 cells 128 against 115 (lanes whose tail moves
+  // to the warps).  TS1 is always faster there: 36 against 293 ms for 4096
+  // cells.  A mechanism with few operations per attempt spends them on the
+  // parts that every lane of the warp repeats: saprc99_mini wins up to 8192
+  // cells (2500 cells: 1.38 against 3.14 ms; 32768: 8.8 against 7.2 ms), one
+  // whose lanes keep their store in registers a few hundred (small_strato: 72
+  // cells 1.8 against 2.7 ms, 4096 cells 6.1 against 3.5; Chapman: 0.51 against
+  // 0.57 ms, 2.1 against 0.67).
   int coop_cells = Mech::TABLE_ATTEMPT ? INT32_MAX : Mech::LU_FMA > 2000 ? 14000 : StoreInfo::kTile ? 10000 : 600;
 };
 

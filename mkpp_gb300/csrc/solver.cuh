@@ -612,7 +612,7 @@ __global__ void __launch_bounds__(32) integrate_coop_kernel(LaunchArgs a) {
 // (by the SM id the hardware reports) integrate the first split_cells cells
 // of the order, the most expensive ones, each on a whole warp from its
 // start, while the blocks on the other SMs run the persistent body over the
-// rest of the order.  A warp finishes a SAPRC99 attempt ~3x sooner than a
+// rest of the order.  A warp finishes a SAPRC99 attempt ~5x sooner than a
 // lane when its SM runs no lanes, so the cells that would set the end of
 // the launch on lanes finish earlier; reserving whole SMs keeps the
 // persistent blocks' FP64 work off those warps' SMs.  Each warp takes the

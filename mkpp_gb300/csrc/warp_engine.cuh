@@ -15,12 +15,14 @@ constexpr int kProgramAhead = 8;
 // steps.
 //
 // Bound by latency: a GB300 warp issues one FP64 instruction per 64 cycles,
-// whatever its active lanes, and any other instruction gets the result ~40
-// cycles later, so a step is an FMA, the store of its result and the loads of
-// the next operands.  Measured on SAPRC99's 2288 steps: 131 cycles a step with
-// up to four warps on an SM and 165 with eight (the FP64 pipe's bound there is
-// 152), against 172 and 204 with a vote for pivots in every step, operand
-// loads under branches and the words of a step each waited for alone.
+// whatever its active lanes, and an FMA whose result anything but the next FMA
+// uses takes 108, so a step is an FMA, the store of its result and the loads of
+// the next operands.  Measured on SAPRC99's 2296 steps, up to four warps on an SM:
+// 164 cycles a step in the LU (5 of them bank conflicts, some 28 the steps with
+// reciprocals, by their number) and 111-120 in the solves, and with eight 209 and 143-150 (the FP64 pipe's
+// bound there is 152); 172 and 204 on average with a vote for pivots in every
+// step, operand loads under branches and the words of a step each waited for
+// alone.
 template <int kPivotEvery>
 struct WarpProgram {
   // Returns false if a reciprocal of this lane met a zero.
