@@ -26,12 +26,12 @@ constexpr size_t kSlots = std::max(std::max(Mech::WARP_SLOTS, Mech::ADJ_COOP_SLO
 
 }  // namespace
 
-// Up to as many cells as a plain integrate, whose lanes take half as long per
-// step; small_strato's tangent, whose lanes walk a program on the global tile,
-// up to more (4325 cells: 11.6 against 15 ms, 8000: 19 against 15; its gradient
-// 11.3 against 9.7 ms, 2000 cells 6.3 against 6.6).
+// Up to as many cells as a plain integrate; register stores longer: small_strato's
+// gradient 6.3 against 6.6 ms for 2000 cells, 11.3 against 9.7 for 4325, and its
+// tangent, whose lanes walk a program on the global tile, 9.6 ms for 4325 cells
+// and 13.5 for 8000 against 14 on lanes.
 bool sweep_on_warps(size_t cells, bool tangent) {
-  constexpr size_t kRegister = Mech::NLU > 20 ? 2000 : 300, kTangent = Mech::NLU > 20 ? 5000 : 300;
+  constexpr size_t kRegister = Mech::NLU > 20 ? 2000 : 300, kTangent = Mech::NLU > 20 ? 8000 : 300;
   const size_t most = coop_cells() == 0 ? 0
                       : StoreInfo::kTile ? (size_t)coop_cells()
                                          : (tangent ? kTangent : kRegister);
