@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(128, 1) eval_cell_jacobian_kernel(size_t n, co
 // cell c), or 0x8000 + a power.
 __device__ __forceinline__ double product(double k, unsigned code, const double* __restrict__ conc, size_t c,
                                           size_t n) {
-  const unsigned short* __restrict__ f = T::factor + (code >> 4);
+  const unsigned short* __restrict__ f = T::factor<> + (code >> 4);
   double v = k;
   for (unsigned i = 0; i < (code & 15u); ++i) {
     const unsigned x = __ldg(f + i);
@@ -87,12 +87,12 @@ __global__ void __launch_bounds__(kRateWarps * 32) eval_rates_kernel(size_t n, c
   const size_t cell = blockIdx.x * (size_t)32 + lane;
   const size_t c = cell < n ? cell : n - 1;
   for (int r = warp; r < Mech::NR; r += kRateWarps)
-    q[r * 32 + lane] = product(__ldg(ktab + c + n * r), T::rate[r], conc, c, n);
+    q[r * 32 + lane] = product(__ldg(ktab + c + n * r), T::rate<>[r], conc, c, n);
   __syncthreads();
   for (int i = warp; i < Mech::NS; i += kRateWarps) {
-    const int begin = T::f_ptr[i], end = T::f_ptr[i + 1];
-    double v = begin < end ? first_term(T::f_coef[begin], q[T::f_term[begin] * 32 + lane]) : 0.0;
-    for (int t = begin + 1; t < end; ++t) v = fma(T::f_coef[t], q[T::f_term[t] * 32 + lane], v);
+    const int begin = T::f_ptr<>[i], end = T::f_ptr<>[i + 1];
+    double v = begin < end ? first_term(T::f_coef<>[begin], q[T::f_term<>[begin] * 32 + lane]) : 0.0;
+    for (int t = begin + 1; t < end; ++t) v = fma(T::f_coef<>[t], q[T::f_term<>[t] * 32 + lane], v);
     if (cell < n) out[cell + n * i] = v;
   }
 }
@@ -107,10 +107,10 @@ __global__ void __launch_bounds__(kWarps * 32) eval_jacobian_kernel(size_t n, co
   const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const size_t cell = blockIdx.x * (size_t)kRow + lane;
   const int col = blockIdx.y;
-  const int first = T::p_ptr[col], count = T::p_ptr[col + 1] - first;
+  const int first = T::p_ptr<>[col], count = T::p_ptr<>[col + 1] - first;
   for (int p = warp; p < count; p += kWarps) {
-    const double* k = ktab + n * T::p_rate[first + p];
-    const unsigned code = T::p_product[first + p];
+    const double* k = ktab + n * T::p_rate<>[first + p];
+    const unsigned code = T::p_product<>[first + p];
 #pragma unroll
     for (int i = 0; i < kCells; ++i) {
       const size_t c = cell + 32 * i < n ? cell + 32 * i : n - 1;
@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(kWarps * 32) eval_jacobian_kernel(size_t n, co
   }
   __syncthreads();
   double* column = out + n * (size_t)Mech::NS * col + cell;
-  const unsigned* entries = T::j_ptr + Mech::NS * col;
+  const unsigned* entries = T::j_ptr<> + Mech::NS * col;
   for (int row = warp; row < Mech::NS; row += kWarps) {
     const unsigned entry = entries[row];
     double v[kCells];
@@ -130,12 +130,12 @@ __global__ void __launch_bounds__(kWarps * 32) eval_jacobian_kernel(size_t n, co
       int t = entry >> 2;
       if (!(entry & 1u) && t < end) {
 #pragma unroll
-        for (int i = 0; i < kCells; ++i) v[i] = first_term(T::j_coef[t], d[T::j_term[t] * kRow + 32 * i + lane]);
+        for (int i = 0; i < kCells; ++i) v[i] = first_term(T::j_coef<>[t], d[T::j_term<>[t] * kRow + 32 * i + lane]);
         ++t;
       }
       for (; t < end; ++t) {
 #pragma unroll
-        for (int i = 0; i < kCells; ++i) v[i] = fma(T::j_coef[t], d[T::j_term[t] * kRow + 32 * i + lane], v[i]);
+        for (int i = 0; i < kCells; ++i) v[i] = fma(T::j_coef<>[t], d[T::j_term<>[t] * kRow + 32 * i + lane], v[i]);
       }
 #pragma unroll
       for (int i = 0; i < kCells; ++i) v[i] = -v[i];

@@ -135,8 +135,16 @@ def _interleave(c, plan, ops, operands, scale):
                 c(f"      S[{out}] = v{out};")
 
 
-def _c_array(c, ctype, name, values):
+# Large tables are variable templates: each of a library's translation units
+# holds those that its own kernels use (as plain arrays all twelve units held
+# every table, and libmkpp_ts1.so was 135 MB).
+PER_USE = "template <int = 0>"
+
+
+def _c_array(c, ctype, name, values, per_use=False):
     vals = [str(v) for v in values] or ["0"]
+    if per_use:
+        c(PER_USE)
     c(f"static __device__ const {ctype} {name}[{len(vals)}] = {{")
     for i in range(0, len(vals), 32):
         c(f"    {', '.join(vals[i:i + 32])},")
@@ -146,6 +154,7 @@ def _c_array(c, ctype, name, values):
 def _c_u64_array(c, name, values):
     vals = list(values) or [0]
     rows = [", ".join(f"0x{v:x}ull" for v in vals[i:i + 8]) for i in range(0, len(vals), 8)]
+    c(PER_USE)
     c(f"alignas(16) static __device__ const unsigned long long {name}[{len(vals)}] = {{")
     for r in rows:
         c(f"    {r},")
@@ -762,7 +771,7 @@ def _emit_warp_sweeps(c, t, sweeps):
         c("  }")
         c("  template <class Run>")
         c(f"  __device__ __forceinline__ static void {step}_coop(double* S, unsigned lane, const Run& run) {{")
-        c(f"    run(S, coop::{name}_sched, coop::{name.upper()}_STEPS, lane);")
+        c(f"    run(S, coop::{name}_sched<>, coop::{name.upper()}_STEPS, lane);")
         c("  }")
 
 
@@ -789,7 +798,7 @@ def _emit_tlm(c, t, tlm, C):
     for (st, j), slot in tlm["cterm"].items():
         cv = C[(st - 1) * (st - 2) // 2 + j - 1]
         c(f"    S[{slot}] = mkpp::divide({_lit(cv)}, h);    // c{st}{j} / h")
-    c("    mkpp::run_program<false>(S, coop::tlm_prog, coop::TLM_OPS);")
+    c("    mkpp::run_program<false>(S, coop::tlm_prog<>, coop::TLM_OPS);")
     c("  }")
 
 
@@ -812,20 +821,22 @@ def _emit_table_adjoint(c, coop):
     c("  __device__ __forceinline__ static void adjoint_step(SA& S, const KA& k, double h) {")
     c("    (void)k;")
     c("    (void)h;")
-    c("    mkpp::run_program<false>(S, coop::adj_prog, coop::ADJ_OPS);")
+    c("    mkpp::run_program<false>(S, coop::adj_prog<>, coop::ADJ_OPS);")
     c("  }")
     c("")
-    c("  // ---- tendencies and Jacobian (table-driven evaluation entries) ----")
+    c("  // ---- tendencies and Jacobian as a program, for host checks of the tables ----")
+    c("#ifndef __CUDACC__")
     c("  // For y in S[Y..]: F(y) into S[F..] and W with 1/(gamma h) = 0, that is")
-    c("  // -J, into the W slots of the LU store.  Walks coop::eval_prog, the")
-    c("  // first stage's partials, W and F code without the factorization.")
+    c("  // -J, into the W slots of the LU store: the first stage's partials, W and F")
+    c("  // code without the factorization.")
     c("  template <class SA, class KA>")
-    c("  __device__ __forceinline__ static void eval_step(SA& S, const KA& k) {")
+    c("  static void eval_step(SA& S, const KA& k) {")
     c("    for (int r = 0; r < NR; ++r) S[KT + r] = k(r);")
     c("    for (int i = 0; i < NCONST; ++i) S[CB + i] = coop::const_val[i];")
     c("    S[CB + 3] = 0.0;  // 1/(gamma h)")
-    c("    mkpp::run_program<false>(S, coop::eval_prog, coop::EVAL_OPS);")
+    c("    mkpp::run_program<false>(S, coop::eval_prog<>, coop::EVAL_OPS);")
     c("  }")
+    c("#endif")
 
 
 def _emit_table_attempt_head(c, coop, C):
@@ -844,7 +855,7 @@ def _emit_table_attempt_head(c, coop, C):
     for (st, j), slot in coop["cterm_slot"].items():
         cv = C[(st - 1) * (st - 2) // 2 + j - 1]
         c(f"    S[{slot}] = mkpp::divide({_lit(cv)}, h);    // c{st}{j} / h")
-    c("    if (!mkpp::run_program<true>(S, coop::attempt_prog, coop::ATTEMPT_OPS)) status |= 1;")
+    c("    if (!mkpp::run_program<true>(S, coop::attempt_prog<>, coop::ATTEMPT_OPS)) status |= 1;")
 
 
 def _emit_coop(c, plan, coop, nv, ns, stages, C, M, E, K0, Y, FS, DY):
@@ -891,7 +902,9 @@ def _emit_coop(c, plan, coop, nv, ns, stages, C, M, E, K0, Y, FS, DY):
         _c_program(t, "ADJ_OPS", "adj_prog", ops)
     if coop["eval_ops"] is not None:
         ops = coop["eval_ops"]
+        t("#ifndef __CUDACC__")
         _c_program(t, "EVAL_OPS", "eval_prog", ops)
+        t("#endif")
     tlm = _tlm_build(plan, nv, stages, coop["A"], C, M, coop["NewF"], K0, Y, Mech_KT, coop["total"])
     tlm_code = _Code()
     _emit_tlm(tlm_code, t, tlm, C)
@@ -921,7 +934,7 @@ def _emit_coop(c, plan, coop, nv, ns, stages, C, M, E, K0, Y, FS, DY):
     c("    // 1/(gamma h) and the c_ij/h, one division of the whole warp.")
     c("    if (lane < T::H_TERMS) S[WCB + 3 + lane] = mkpp::divide(T::h_num[lane], lane == 0 ? GAMMA * h : h);")
     c("    __syncwarp();")
-    c("    const bool ok = run(S, T::sched, T::stage_step[NSTAGE], lane);")
+    c("    const bool ok = run(S, T::sched<>, T::stage_step[NSTAGE], lane);")
     c("    if (__any_sync(0xffffffffu, !ok)) status |= 1;")
     c("  }")
     c("")
@@ -1031,7 +1044,7 @@ def _eval_tables(plan) -> str:
                               ("p_rate", "unsigned short", p_rate), ("p_product", "unsigned", p_product),
                               ("j_ptr", "unsigned", j_ptr), ("j_term", "unsigned short", j_term),
                               ("j_coef", "double", j_coef)):
-        _c_array(t, ctype, name, vals)
+        _c_array(t, ctype, name, vals, per_use=True)
     t("}  // namespace eval")
     t("")
     return t.text()
