@@ -6,17 +6,13 @@ namespace mkpp_tu {
 
 namespace {
 
-// Launches `kernel` with one warp per block, as many as the cells and the
-// shared memory of the SMs allow.
+// Launches `kernel` with a block of one warp per cell.
 template <class Kernel, class... Args>
-int launch_warps(Kernel kernel, size_t slots, int cells, unsigned* next, cudaStream_t stream, const Args&... args) {
+int launch_warps(Kernel kernel, size_t slots, int cells, cudaStream_t stream, const Args&... args) {
   const size_t smem = slots * sizeof(double);
-  int per_sm = 0;
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 32, smem) != cudaSuccess || per_sm < 1)
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     return MKPP_ERROR_DEVICE;
-  if (cudaMemsetAsync(next, 0, sizeof(unsigned), stream) != cudaSuccess) return MKPP_ERROR_DEVICE;
-  kernel<<<std::min(cells, per_sm * sm_count()), 32, smem, stream>>>(args...);
+  kernel<<<cells, 32, smem, stream>>>(args...);
   return cudaGetLastError() == cudaSuccess ? MKPP_SUCCESS : MKPP_ERROR_DEVICE;
 }
 
@@ -38,19 +34,16 @@ bool sweep_on_warps(size_t cells, bool tangent) {
   return kSlots * sizeof(double) <= kMaxSmem && cells <= most;
 }
 
-int launch_checkpoint_coop(mkpp::LaunchArgs a, const mkpp::CheckpointArgs& ck, unsigned* next, cudaStream_t stream) {
-  a.coop_next = next;
-  return launch_warps(mkpp::checkpoint_coop_kernel<Mech>, Mech::WARP_SLOTS, a.ncells, next, stream, a, ck);
+int launch_checkpoint_coop(const mkpp::LaunchArgs& a, const mkpp::CheckpointArgs& ck, cudaStream_t stream) {
+  return launch_warps(mkpp::checkpoint_coop_kernel<Mech>, Mech::WARP_SLOTS, a.ncells, stream, a, ck);
 }
 
-int launch_adjoint_coop(const mkpp::AdjointArgs& a, const mkpp::CheckpointArgs& ck, unsigned* next,
-                        cudaStream_t stream) {
-  return launch_warps(mkpp::adjoint_coop_kernel<Mech>, Mech::ADJ_COOP_SLOTS, a.ncells, next, stream, a, ck, next);
+int launch_adjoint_coop(const mkpp::AdjointArgs& a, const mkpp::CheckpointArgs& ck, cudaStream_t stream) {
+  return launch_warps(mkpp::adjoint_coop_kernel<Mech>, Mech::ADJ_COOP_SLOTS, a.ncells, stream, a, ck);
 }
 
-int launch_tangent_coop(const mkpp::TangentArgs& a, const mkpp::CheckpointArgs& ck, unsigned* next,
-                        cudaStream_t stream) {
-  return launch_warps(mkpp::tangent_coop_kernel<Mech>, Mech::TLM_COOP_SLOTS, a.ncells, next, stream, a, ck, next);
+int launch_tangent_coop(const mkpp::TangentArgs& a, const mkpp::CheckpointArgs& ck, cudaStream_t stream) {
+  return launch_warps(mkpp::tangent_coop_kernel<Mech>, Mech::TLM_COOP_SLOTS, a.ncells, stream, a, ck);
 }
 
 }  // namespace mkpp_tu
