@@ -36,6 +36,19 @@ inline int sm_count() {
   return sms;
 }
 
+// Dynamic shared memory of a block on sm_103.
+constexpr size_t kMaxSmem = 227 * 1024;
+
+// Lets `kernel` use `bytes` of dynamic shared memory.  False if it cannot, with
+// no error left behind for the next launch's check.
+template <class Kernel>
+bool allow_smem(Kernel kernel, size_t bytes) {
+  if (bytes > kMaxSmem) return false;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess) return true;
+  (void)cudaGetLastError();
+  return false;
+}
+
 inline mkpp::LaunchArgs make_args(size_t cells, double* conc, const double* ktab, int steps, double dt, double seed,
                                   int max_attempts, int* status, int* accepted, int* rejected) {
   mkpp::LaunchArgs a;

@@ -7,11 +7,12 @@ namespace mkpp_tu {
 
 int coop_resident_blocks(size_t smem) {
   int per_sm = 0;
-  if (cudaFuncSetAttribute(mkpp::integrate_coop_kernel<Mech>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)smem) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mkpp::integrate_coop_kernel<Mech>, 32, smem) !=
-          cudaSuccess)
+  if (!allow_smem(mkpp::integrate_coop_kernel<Mech>, smem)) return 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mkpp::integrate_coop_kernel<Mech>, 32, smem) !=
+      cudaSuccess) {
+    (void)cudaGetLastError();
     return 0;
+  }
   return per_sm;
 }
 

@@ -10,14 +10,11 @@ namespace {
 template <class Kernel, class... Args>
 int launch_warps(Kernel kernel, size_t slots, int cells, cudaStream_t stream, const Args&... args) {
   const size_t smem = slots * sizeof(double);
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return MKPP_ERROR_DEVICE;
+  if (!allow_smem(kernel, smem)) return MKPP_ERROR_DEVICE;
   kernel<<<cells, 32, smem, stream>>>(args...);
   return cudaGetLastError() == cudaSuccess ? MKPP_SUCCESS : MKPP_ERROR_DEVICE;
 }
 
-// A block's shared memory on sm_103.
-constexpr size_t kMaxSmem = 227 * 1024;
 constexpr size_t kSlots = std::max(std::max(Mech::WARP_SLOTS, Mech::ADJ_COOP_SLOTS), Mech::TLM_COOP_SLOTS);
 
 }  // namespace
