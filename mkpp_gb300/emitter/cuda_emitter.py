@@ -49,6 +49,28 @@ def _k_text(expr: str) -> str:
     return expr
 
 
+# Texts that mkpp::Num (csrc/mkpp_device.cuh) can stand in for a double in:
+# numbers, the four operators, and these names.
+_NUM_NAMES = {"T", "RHO", "RH", "CLW", "P", "FIX", "exp", "log", "sqrt", "fabs", "pow", "M_LN10"}
+
+
+def _takes_num(expr: str) -> bool:
+    text = re.sub(r"(?<![\w.])(?:\d+\.?\d*|\.\d+)(?:[eE][+-]?\d+)?(?![\w.])", "0", expr)
+    names = set(re.findall(r"[A-Za-z_]\w*", text))
+    return (names <= _NUM_NAMES and not re.search(r"[^\w\s+\-*/(),]", text)
+            and not re.search(r"(?:^|[-+*/(,])\s*\+", text))
+
+
+def _k_value(expr: str) -> str:
+    """The rate constant `expr` of rate_constants_part().  What only a double
+    can do (a comparison, fmin, cbrt, ...) is evaluated on doubles."""
+    expr = _k_text(expr)
+    if _takes_num(expr):
+        return f"mkpp::value({expr})"
+    return (f"[&](double T, double RHO, double RH, double CLW) -> double {{ (void)T; (void)RHO; (void)RH; (void)CLW; "
+            f"return {expr}; }}(mkpp::value(T), mkpp::value(RHO), mkpp::value(RH), mkpp::value(CLW))")
+
+
 class _Code:
     def __init__(self):
         self.lines: list[str] = []
@@ -1357,7 +1379,8 @@ def emit_mechanism(plan: ReducedPlan, table: bool | None = None) -> str:
     c("  // rate kernel gives to different blocks.")
     parts = _rate_parts(plan.reactions)
     c(f"  static constexpr int RATE_PARTS = {len(parts)};")
-    c("  // V is double, or mkpp::Num, whose divisions take the integer pipes.")
+    c("  // V is double, or mkpp::Num, whose divisions take the integer pipes; texts")
+    c("  // that Num cannot take are evaluated on doubles either way.")
     c("  template <class PA, class FA, class KO, class V>")
     c("  __device__ __forceinline__ static void rate_constants_part(int part, const PA& P, const FA& FIX, V T, V RHO,")
     c("                                                           V RH, V CLW, KO& k) {")
@@ -1366,7 +1389,7 @@ def emit_mechanism(plan: ReducedPlan, table: bool | None = None) -> str:
     for i, part in enumerate(parts):
         c(f"      case {i}:")
         for r in part:
-            c(f"        k.set({r.index}, mkpp::value({_k_text(r.k)}));")
+            c(f"        k.set({r.index}, {_k_value(r.k)});")
         c("        break;")
     c("    }")
     c("  }")
