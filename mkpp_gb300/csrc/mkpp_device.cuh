@@ -168,7 +168,11 @@ __device__ __forceinline__ double max_abs(double x, double y) {
 // two flags (emitter/warp_schedule.py):
 //   a: 1 negate the product | b, c: 1 the lane's previous result instead |
 //   out: 1 store nothing, 2 reciprocal.
+// A program with slots beyond 14 bits has words of 128, four 32-bit fields.
 // ---------------------------------------------------------------------------
+struct alignas(16) WideWord {
+  unsigned long long lo, hi;
+};
 struct ProgramWord {
   unsigned lo, hi;
   __device__ __forceinline__ ProgramWord(unsigned long long w) : lo((unsigned)w), hi((unsigned)(w >> 32)) {}
@@ -181,7 +185,27 @@ struct ProgramWord {
   __device__ __forceinline__ unsigned b() const { return lo >> 18; }
   __device__ __forceinline__ unsigned c() const { return (hi >> 2) & 0x3fffu; }
   __device__ __forceinline__ unsigned out() const { return hi >> 18; }
+  __device__ __forceinline__ unsigned last() const { return hi; }  // the word's end with the out field
 };
+struct WideProgramWord {
+  unsigned fa, fb, fc, fo;
+  __device__ __forceinline__ WideProgramWord(const WideWord& w)
+      : fa((unsigned)w.lo), fb((unsigned)(w.lo >> 32)), fc((unsigned)w.hi), fo((unsigned)(w.hi >> 32)) {}
+  __device__ __forceinline__ unsigned negate() const { return fa << 31; }
+  __device__ __forceinline__ bool prev_b() const { return fb & 1u; }
+  __device__ __forceinline__ bool prev_c() const { return fc & 1u; }
+  __device__ __forceinline__ bool stores() const { return !(fo & 1u); }
+  __device__ __forceinline__ bool reciprocal() const { return fo & 2u; }
+  __device__ __forceinline__ unsigned a() const { return fa >> 2; }
+  __device__ __forceinline__ unsigned b() const { return fb >> 2; }
+  __device__ __forceinline__ unsigned c() const { return fc >> 2; }
+  __device__ __forceinline__ unsigned out() const { return fo >> 2; }
+  __device__ __forceinline__ unsigned last() const { return fo; }
+};
+__device__ __forceinline__ ProgramWord program_word(unsigned long long w) { return ProgramWord(w); }
+__device__ __forceinline__ WideProgramWord program_word(const WideWord& w) { return WideProgramWord(w); }
+__device__ __forceinline__ unsigned long long load_word(const unsigned long long* p) { return __ldg(p); }
+__device__ __forceinline__ WideWord load_word(const WideWord* p) { return WideWord{__ldg(&p->lo), __ldg(&p->hi)}; }
 
 __device__ __forceinline__ double flip_sign(double x, unsigned sign) {
   return __longlong_as_double(__double_as_longlong(x) ^ ((long long)sign << 32));
@@ -192,17 +216,17 @@ __device__ __forceinline__ double flip_sign(double x, unsigned sign) {
 // this one's result is stored (what it reads of that comes from the register).
 // Returns false if a reciprocal met a zero; a program without pivots says so,
 // which keeps the division out of its loop.
-template <bool kPivots, class SA>
-__device__ __forceinline__ bool run_program(SA& S, const unsigned long long* __restrict__ prog, int ops) {
+template <bool kPivots, class SA, class Word>
+__device__ __forceinline__ bool run_program(SA& S, const Word* __restrict__ prog, int ops) {
   double prev = 0.0;
   bool ok = true;
-  unsigned long long now = __ldg(prog), next = __ldg(prog + (ops > 1 ? 1 : 0));
-  double A = S[ProgramWord(now).a()], B = S[ProgramWord(now).b()], C = S[ProgramWord(now).c()];
+  Word now = load_word(prog), next = load_word(prog + (ops > 1 ? 1 : 0));
+  double A = S[program_word(now).a()], B = S[program_word(now).b()], C = S[program_word(now).c()];
 #pragma unroll 4
   for (int n = 0; n < ops; ++n) {
-    const ProgramWord w(now), following(next);
+    const auto w = program_word(now), following = program_word(next);
     now = next;
-    next = __ldg(prog + (n + 2 < ops ? n + 2 : ops - 1));
+    next = load_word(prog + (n + 2 < ops ? n + 2 : ops - 1));
     const double a = flip_sign(A, w.negate()), b = w.prev_b() ? prev : B, c = w.prev_c() ? prev : C;
     A = S[following.a()];
     B = S[following.b()];

@@ -9,10 +9,58 @@ namespace mkpp {
 
 constexpr int kProgramAhead = 8;
 
+// What the loop below takes from the words of a program: the byte offsets of
+// the slots, and how the words of a group of steps lie in memory.
+template <class Word>
+struct StepWords;
+
+// 64-bit words, two steps' words of a lane side by side.  A field (slot * 4 +
+// flags), shifted to slot * 8, is a byte offset.
+template <>
+struct StepWords<unsigned long long> {
+  typedef unsigned long long Word;
+  static constexpr unsigned kIdle = 0x10000u;  // last field and its half word: nothing to store
+  __device__ __forceinline__ static void fetch(const ulonglong2* __restrict__ words, int g, Word* to) {
+    constexpr int kPairs = kProgramAhead / 2;
+#pragma unroll
+    for (int j = 0; j < kPairs; ++j) {
+      const ulonglong2 v = __ldg(words + ((size_t)g * kPairs + j) * 32);
+      to[2 * j] = v.x;
+      to[2 * j + 1] = v.y;
+    }
+  }
+  __device__ __forceinline__ static unsigned a(Word v) { return ((unsigned)v << 1) & 0x1fff8u; }
+  __device__ __forceinline__ static unsigned b(Word v) { return ((unsigned)v >> 15) & 0x1fff8u; }
+  __device__ __forceinline__ static unsigned c(Word v) { return ((unsigned)(v >> 32) << 1) & 0x1fff8u; }
+  __device__ __forceinline__ static unsigned last(Word v) { return (unsigned)(v >> 32); }
+  __device__ __forceinline__ static unsigned out(unsigned last) { return (last >> 15) & 0x1fff8u; }
+  __device__ __forceinline__ static bool stores(unsigned last) { return !(last & 0x10000u); }
+  __device__ __forceinline__ static bool reciprocal(unsigned last) { return last & 0x20000u; }
+};
+
+// 128-bit words.
+template <>
+struct StepWords<WideWord> {
+  static constexpr unsigned kIdle = 1u;
+  __device__ __forceinline__ static void fetch(const ulonglong2* __restrict__ words, int g, WideWord* to) {
+#pragma unroll
+    for (int j = 0; j < kProgramAhead; ++j) {
+      const ulonglong2 v = __ldg(words + ((size_t)g * kProgramAhead + j) * 32);
+      to[j] = WideWord{v.x, v.y};
+    }
+  }
+  __device__ __forceinline__ static unsigned a(const WideWord& v) { return WideProgramWord(v).a() * 8u; }
+  __device__ __forceinline__ static unsigned b(const WideWord& v) { return WideProgramWord(v).b() * 8u; }
+  __device__ __forceinline__ static unsigned c(const WideWord& v) { return WideProgramWord(v).c() * 8u; }
+  __device__ __forceinline__ static unsigned last(const WideWord& v) { return (unsigned)(v.hi >> 32); }
+  __device__ __forceinline__ static unsigned out(unsigned last) { return (last >> 2) * 8u; }
+  __device__ __forceinline__ static bool stores(unsigned last) { return !(last & 1u); }
+  __device__ __forceinline__ static bool reciprocal(unsigned last) { return last & 2u; }
+};
+
 // One warp runs `steps` steps (a multiple of kProgramAhead, the last one idle)
-// of 32 words, a lane per word, two steps' words of a lane side by side, on
-// one store that the warp shares; reciprocals only in the last of kPivotEvery
-// steps.
+// of 32 words, a lane per word, on one store that the warp shares; reciprocals
+// only in the last of kPivotEvery steps.
 //
 // Bound by latency: a GB300 warp issues one FP64 instruction per 64 cycles,
 // whatever its active lanes, and an FMA whose result anything but the next FMA
@@ -26,37 +74,27 @@ constexpr int kProgramAhead = 8;
 template <int kPivotEvery>
 struct WarpProgram {
   // Returns false if a reciprocal of this lane met a zero.
-  __device__ __forceinline__ bool operator()(double* S, const unsigned long long* __restrict__ prog, int steps,
-                                             unsigned lane) const {
-    constexpr int kPairs = kProgramAhead / 2;
+  template <class Word>
+  __device__ __forceinline__ bool operator()(double* S, const Word* __restrict__ prog, int steps, unsigned lane) const {
+    typedef StepWords<Word> Words;
     const ulonglong2* __restrict__ words = reinterpret_cast<const ulonglong2*>(prog) + lane;
     char* const base = reinterpret_cast<char*>(S);
     const int groups = steps / kProgramAhead;
-    unsigned long long w[kProgramAhead];
-    auto fetch = [&](int g, unsigned long long* to) {
-#pragma unroll
-      for (int j = 0; j < kPairs; ++j) {
-        const ulonglong2 v = __ldg(words + ((size_t)g * kPairs + j) * 32);
-        to[2 * j] = v.x;
-        to[2 * j + 1] = v.y;
-      }
-    };
-    // A field (slot * 4 + flags), shifted to slot * 8, is its byte offset.
-    auto at = [&](unsigned offset) { return reinterpret_cast<double*>(base + (offset & 0x1fff8u)); };
+    Word w[kProgramAhead];
+    auto at = [&](unsigned offset) { return reinterpret_cast<double*>(base + offset); };
     double A, B, C, prev = 0.0;
-    auto load = [&](unsigned long long v) {
-      const unsigned lo = (unsigned)v, hi = (unsigned)(v >> 32);
-      A = flip_sign(*at(lo << 1), lo << 31);
-      B = *at(lo >> 15);
-      C = *at(hi << 1);
+    auto load = [&](Word v) {
+      A = flip_sign(*at(Words::a(v)), program_word(v).negate());
+      B = *at(Words::b(v));
+      C = *at(Words::c(v));
     };
-    unsigned before = 0x10000u;  // the previous step's high word: nothing to store yet
+    unsigned before = Words::kIdle;  // the previous step's last field: nothing to store yet
     bool ok = true;
     // One group of steps; only some groups hold pivots.
-    auto run = [&](auto pivots, unsigned long long first_after) {
+    auto run = [&](auto pivots, Word first_after) {
 #pragma unroll
       for (int j = 0; j < kProgramAhead; ++j) {
-        const ProgramWord p(w[j]);
+        const auto p = program_word(w[j]);
         const double b = p.prev_b() ? prev : B;
         const double c = p.prev_c() ? prev : C;
         double v = fma(A, b, c);
@@ -67,29 +105,29 @@ struct WarpProgram {
             v = p.reciprocal() ? r : v;
           }
         }
-        if (!(before & 0x10000u)) *at(before >> 15) = prev;
+        if (Words::stores(before)) *at(Words::out(before)) = prev;
         __syncwarp();
         load(j + 1 < kProgramAhead ? w[j + 1] : first_after);
         prev = v;
-        before = p.hi;
+        before = p.last();
       }
     };
-    fetch(0, w);
+    Words::fetch(words, 0, w);
     load(w[0]);
     for (int g = 0; g < groups; ++g) {
-      unsigned long long next[kProgramAhead];
-      fetch(g + 1 < groups ? g + 1 : g, next);
+      Word next[kProgramAhead];
+      Words::fetch(words, g + 1 < groups ? g + 1 : g, next);
       unsigned any = 0;
 #pragma unroll
-      for (int j = 0; j < kProgramAhead; ++j) any |= (unsigned)(w[j] >> 32);
-      if (__any_sync(0xffffffffu, any & 0x20000u))
+      for (int j = 0; j < kProgramAhead; ++j) any |= Words::last(w[j]);
+      if (__any_sync(0xffffffffu, Words::reciprocal(any)))
         run(std::true_type(), next[0]);
       else
         run(std::false_type(), next[0]);
 #pragma unroll
       for (int j = 0; j < kProgramAhead; ++j) w[j] = next[j];
     }
-    if (!(before & 0x10000u)) *at(before >> 15) = prev;
+    if (Words::stores(before)) *at(Words::out(before)) = prev;
     __syncwarp();
     return ok;
   }

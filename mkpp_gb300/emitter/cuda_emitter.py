@@ -173,21 +173,33 @@ def _c_array(c, ctype, name, values, per_use=False):
     c("};")
 
 
-def _c_u64_array(c, name, values):
-    vals = list(values) or [0]
-    rows = [", ".join(f"0x{v:x}ull" for v in vals[i:i + 8]) for i in range(0, len(vals), 8)]
+def _c_words(c, name, words, bits):
+    """Table of program words (csrc/mkpp_device.cuh: one 64-bit number each, or
+    mkpp::WideWord)."""
+    vals = list(words) or [0]
     c(PER_USE)
-    c(f"alignas(16) static __device__ const unsigned long long {name}[{len(vals)}] = {{")
-    for r in rows:
-        c(f"    {r},")
+    if bits == warp_schedule.WIDE:
+        low = (1 << 64) - 1
+        c(f"static __device__ const mkpp::WideWord {name}[{len(vals)}] = {{")
+        for i in range(0, len(vals), 4):
+            c(f"    {', '.join(f'{{0x{v & low:x}ull, 0x{v >> 64:x}ull}}' for v in vals[i:i + 4])},")
+    else:
+        c(f"alignas(16) static __device__ const unsigned long long {name}[{len(vals)}] = {{")
+        for i in range(0, len(vals), 8):
+            c(f"    {', '.join(f'0x{v:x}ull' for v in vals[i:i + 8])},")
     c("};")
+
+
+def _field_bits(*programs):
+    return warp_schedule.WIDE if warp_schedule.is_wide(*programs) else warp_schedule.NARROW
 
 
 def _c_program(c, count, name, ops):
     """A program of one thread: its words and their number."""
-    words = warp_schedule.encode(ops, warp_schedule.sequential(ops), lanes=1)
+    bits = _field_bits(ops)
+    words = warp_schedule.encode(ops, warp_schedule.sequential(ops), 1, bits)
     c(f"constexpr int {count} = {len(words)};")
-    _c_u64_array(c, name, words)
+    _c_words(c, name, words, bits)
 
 
 def _shifted(ops, first, by):
@@ -783,7 +795,8 @@ def _emit_warp_sweeps(c, t, sweeps):
         c(f"  static constexpr int {name} = {slot};")
     for name, sw in sweeps.items():
         t(f"constexpr int {name.upper()}_STEPS = {len(sw['steps'])};")
-        _c_u64_array(t, f"{name}_sched", warp_schedule.encode(sw["ops"], sw["steps"]))
+        bits = _field_bits(sw["ops"])
+        _c_words(t, f"{name}_sched", warp_schedule.encode(sw["ops"], sw["steps"], bits=bits), bits)
         _c_array(t, "double", f"{name}_lit", [_lit(v) for v in sw["extra"]])
         step = {"adj": "adjoint", "tlm": "tangent"}[name]
         c(f"  // adjoint_step() and tlm_step() after stages_coop() for the same step." if name == "adj" else "")
@@ -912,10 +925,11 @@ def _emit_coop(c, plan, coop, nv, ns, stages, C, M, E, K0, Y, FS, DY):
     assert list(cterm_slot.values()) == [CB + 4 + i for i in range(len(cterm_slot))]
     t(f"constexpr int H_TERMS = {len(nums)};")
     t(f"static __device__ const double h_num[{len(nums)}] = {{{', '.join(nums)}}};")
+    bits = _field_bits(*coop["warp"])
     words = []
     for ops, st_ in zip(coop["warp"], sched):
-        words += warp_schedule.encode(ops, st_)
-    _c_u64_array(t, "sched", words)
+        words += warp_schedule.encode(ops, st_, bits=bits)
+    _c_words(t, "sched", words, bits)
     if coop["seq_ops"] is not None:
         ops = coop["seq_ops"]
         _c_program(t, "ATTEMPT_OPS", "attempt_prog", ops)

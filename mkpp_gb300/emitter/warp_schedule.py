@@ -46,7 +46,8 @@ two flags below it, so that a field is a byte offset after one shift:
   bits 32-47  c: slot * 4 + (the lane's previous result instead)
   bits 48-63  out: slot * 4 + 2 * (reciprocal of b) + (store nothing)
 Storing nothing is an idle lane, or a result that only the lane's next
-operation reads.
+operation reads.  A program that addresses a slot beyond 14 bits (``is_wide``;
+none of the shipped ones) has words of four 32-bit fields, laid out alike.
 """
 
 from __future__ import annotations
@@ -56,8 +57,13 @@ import heapq
 FMA, RCP = 1, 2
 LANES = 32
 AHEAD = 8             # steps per unrolled group of the device loop
-IDLE = 1 << 48        # word of an idle lane
+NARROW, WIDE = 16, 32  # bits of a word's field
 PREV = -1             # operand: the lane's previous result
+
+
+def is_wide(*programs) -> bool:
+    """Whether the programs' slots need the wide words."""
+    return any(x >= 1 << (NARROW - 2) for ops in programs for op in ops for x in op[1:5])
 
 
 class Program:
@@ -340,13 +346,14 @@ def sequential(ops) -> list[list[int]]:
     return steps
 
 
-def encode(ops, steps, lanes: int = LANES) -> list[int]:
-    """steps x lanes words (a step lists the operations of its lanes, None or
+def encode(ops, steps, lanes: int = LANES, bits: int = NARROW) -> list[int]:
+    """steps x lanes words with fields of `bits` (a step lists the operations of its lanes, None or
     missing for an idle lane).  An operand whose writer is the lane's
     previous operation, one step before, is taken from the lane's register,
     and a result that nothing else reads is not stored.  With several lanes
-    an odd number of steps is filled up with an idle one, and two steps'
-    words of a lane are side by side."""
+    and narrow words an odd number of steps is filled up with an idle one, and
+    two steps' words of a lane are side by side."""
+    idle = 1 << 3 * bits
     where = {}
     for s, row in enumerate(steps):
         for q, i in enumerate(row):
@@ -375,27 +382,28 @@ def encode(ops, steps, lanes: int = LANES) -> list[int]:
     for i in last.values():
         stored[i] = True
     rows = []
-    for row in list(steps) + [[]] * (len(steps) % 2 if lanes > 1 else 0):
-        line = [IDLE] * lanes
+    pairs = lanes > 1 and bits == NARROW
+    for row in list(steps) + [[]] * (len(steps) % 2 if pairs else 0):
+        line = [idle] * lanes
         for q, i in enumerate(row):
             if i is None:
                 continue
             kind, out, _, _, _, neg = ops[i]
             a, b, c = fields[i]
-            assert all(PREV <= x < 1 << 14 for x in (out, a, b, c)) and a >= 0
-            lo = (a << 2 | bool(neg)) | (max(b, 0) << 2 | (b == PREV)) << 16
-            hi = (max(c, 0) << 2 | (c == PREV)) | (out << 2 | (kind == RCP) << 1 | (not stored[i])) << 16
-            line[q] = lo | hi << 32
+            assert all(PREV <= x < 1 << (bits - 2) for x in (out, a, b, c)) and a >= 0, "a slot exceeds its field"
+            lo = (a << 2 | bool(neg)) | (max(b, 0) << 2 | (b == PREV)) << bits
+            hi = (max(c, 0) << 2 | (c == PREV)) | (out << 2 | (kind == RCP) << 1 | (not stored[i])) << bits
+            line[q] = lo | hi << 2 * bits
         rows.append(line)
-    if lanes == 1:
-        return [line[0] for line in rows]
+    if not pairs:
+        return [word for line in rows for word in line]
     return [line[q] for s in range(0, len(rows), 2) for q in range(lanes) for line in rows[s:s + 2]]
 
 
-def decode(word: int) -> tuple[int, int, int, int, int, int]:
+def decode(word: int, bits: int = NARROW) -> tuple[int, int, int, int, int, int]:
     """(kind, out, a, b, c, neg) of one word; kind 0 for a lane that stores
     nothing, operand -1 for the lane's previous result."""
-    a, b, c, out = ((word >> 16 * f) & 0xFFFF for f in range(4))
+    a, b, c, out = ((word >> bits * f) & ((1 << bits) - 1) for f in range(4))
     if out & 1:
         return 0, out >> 2, 0, 0, 0, 0
     b_, c_ = (PREV if x & 1 else x >> 2 for x in (b, c))
