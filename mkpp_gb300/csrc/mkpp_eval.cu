@@ -12,6 +12,9 @@
 // matrix, wrote W and flipped its sign through tables of slot positions on the
 // stack, took 92.8 ms for SAPRC99's 20000 cells (1.08 GB); this takes 0.23 ms.
 // TS1, 1001 cells: 4.5 -> 0.11 ms, the tendencies 3.1 -> 0.06 ms.
+//
+// Rates (or partials of a column) that 32 cells have too many of for a block's
+// shared memory, above 908, are multiplied out again for each term.
 #include "capi_common.cuh"
 
 using namespace mkpp_tu;
@@ -22,7 +25,8 @@ namespace T = MKPP_MECH_NS::eval;
 
 constexpr int kWarps = 8;       // of a block, one column of the Jacobian
 constexpr int kRateWarps = 16;  // of a block, all rates and tendencies
-constexpr size_t kRatesSmem = (size_t)Mech::NR * 32 * sizeof(double);
+constexpr size_t kRatesSmem = (size_t)T::RATES * 32 * sizeof(double);
+constexpr bool kStageRates = kRatesSmem <= kMaxSmem;
 constexpr size_t kDefaultSmem = 48 * 1024;
 
 // State accessor over a cell's row of the (species x cells) array.
@@ -60,14 +64,14 @@ __global__ void __launch_bounds__(128, 1) eval_cell_jacobian_kernel(size_t n, co
 }
 
 // k times the coded factors, left to right: species (their concentrations in
-// cell c), or 0x8000 + a power.
+// cell c), or POWER + a number.
 __device__ __forceinline__ double product(double k, unsigned code, const double* __restrict__ conc, size_t c,
                                           size_t n) {
-  const unsigned short* __restrict__ f = T::factor<> + (code >> 4);
+  const auto* __restrict__ f = T::factor<> + (code >> T::LEN_BITS);
   double v = k;
-  for (unsigned i = 0; i < (code & 15u); ++i) {
+  for (unsigned i = 0; i < (code & ((1u << T::LEN_BITS) - 1u)); ++i) {
     const unsigned x = __ldg(f + i);
-    v *= (x & 0x8000u) ? (double)(x & 0x7fffu) : __ldg(conc + c + n * x);
+    v *= (x & T::POWER) ? (double)(x & (T::POWER - 1u)) : __ldg(conc + c + n * x);
   }
   return v;
 }
@@ -86,19 +90,28 @@ __global__ void __launch_bounds__(kRateWarps * 32) eval_rates_kernel(size_t n, c
   const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const size_t cell = blockIdx.x * (size_t)32 + lane;
   const size_t c = cell < n ? cell : n - 1;
-  for (int r = warp; r < Mech::NR; r += kRateWarps)
-    q[r * 32 + lane] = product(__ldg(ktab + c + n * r), T::rate<>[r], conc, c, n);
-  __syncthreads();
+  auto product_of = [&](int r) { return product(__ldg(ktab + c + n * r), T::rate<>[r], conc, c, n); };
+  if constexpr (kStageRates) {
+    for (int r = warp; r < T::RATES; r += kRateWarps) q[r * 32 + lane] = product_of(r);
+    __syncthreads();
+  }
+  auto rate = [&](int r) {
+    if constexpr (kStageRates)
+      return q[r * 32 + lane];
+    else
+      return product_of(r);
+  };
   for (int i = warp; i < Mech::NS; i += kRateWarps) {
     const int begin = T::f_ptr<>[i], end = T::f_ptr<>[i + 1];
-    double v = begin < end ? first_term(T::f_coef<>[begin], q[T::f_term<>[begin] * 32 + lane]) : 0.0;
-    for (int t = begin + 1; t < end; ++t) v = fma(T::f_coef<>[t], q[T::f_term<>[t] * 32 + lane], v);
+    double v = begin < end ? first_term(T::f_coef<>[begin], rate(T::f_term<>[begin])) : 0.0;
+    for (int t = begin + 1; t < end; ++t) v = fma(T::f_coef<>[t], rate(T::f_term<>[t]), v);
     if (cell < n) out[cell + n * i] = v;
   }
 }
 
-// Column blockIdx.y of the Jacobian of 32 * kCells cells, kCells per lane.
-template <int kCells>
+// Column blockIdx.y of the Jacobian of 32 * kCells cells, kCells per lane, its
+// partials in shared memory if kStage.
+template <int kCells, bool kStage>
 __global__ void __launch_bounds__(kWarps * 32) eval_jacobian_kernel(size_t n, const double* __restrict__ conc,
                                                                    const double* __restrict__ ktab,
                                                                    double* __restrict__ out) {
@@ -108,16 +121,23 @@ __global__ void __launch_bounds__(kWarps * 32) eval_jacobian_kernel(size_t n, co
   const size_t cell = blockIdx.x * (size_t)kRow + lane;
   const int col = blockIdx.y;
   const int first = T::p_ptr<>[col], count = T::p_ptr<>[col + 1] - first;
-  for (int p = warp; p < count; p += kWarps) {
-    const double* k = ktab + n * T::p_rate<>[first + p];
-    const unsigned code = T::p_product<>[first + p];
+  auto product_of = [&](int p, int i) {
+    const size_t c = cell + 32 * i < n ? cell + 32 * i : n - 1;
+    return product(__ldg(ktab + n * T::p_rate<>[first + p] + c), T::p_product<>[first + p], conc, c, n);
+  };
+  if constexpr (kStage) {
+    for (int p = warp; p < count; p += kWarps) {
 #pragma unroll
-    for (int i = 0; i < kCells; ++i) {
-      const size_t c = cell + 32 * i < n ? cell + 32 * i : n - 1;
-      d[p * kRow + 32 * i + lane] = product(__ldg(k + c), code, conc, c, n);
+      for (int i = 0; i < kCells; ++i) d[p * kRow + 32 * i + lane] = product_of(p, i);
     }
+    __syncthreads();
   }
-  __syncthreads();
+  auto partial = [&](int p, int i) {
+    if constexpr (kStage)
+      return d[p * kRow + 32 * i + lane];
+    else
+      return product_of(p, i);
+  };
   double* column = out + n * (size_t)Mech::NS * col + cell;
   const unsigned* entries = T::j_ptr<> + Mech::NS * col;
   for (int row = warp; row < Mech::NS; row += kWarps) {
@@ -130,12 +150,12 @@ __global__ void __launch_bounds__(kWarps * 32) eval_jacobian_kernel(size_t n, co
       int t = entry >> 2;
       if (!(entry & 1u) && t < end) {
 #pragma unroll
-        for (int i = 0; i < kCells; ++i) v[i] = first_term(T::j_coef<>[t], d[T::j_term<>[t] * kRow + 32 * i + lane]);
+        for (int i = 0; i < kCells; ++i) v[i] = first_term(T::j_coef<>[t], partial(T::j_term<>[t], i));
         ++t;
       }
       for (; t < end; ++t) {
 #pragma unroll
-        for (int i = 0; i < kCells; ++i) v[i] = fma(T::j_coef<>[t], d[T::j_term<>[t] * kRow + 32 * i + lane], v[i]);
+        for (int i = 0; i < kCells; ++i) v[i] = fma(T::j_coef<>[t], partial(T::j_term<>[t], i), v[i]);
       }
 #pragma unroll
       for (int i = 0; i < kCells; ++i) v[i] = -v[i];
@@ -148,12 +168,12 @@ __global__ void __launch_bounds__(kWarps * 32) eval_jacobian_kernel(size_t n, co
 
 template <int kCells>
 int launch_jacobian(size_t n, const double* conc, const double* ktab, double* out, cudaStream_t stream) {
-  constexpr size_t kSmem = (size_t)(T::MAX_PARTIALS > 0 ? T::MAX_PARTIALS : 1) * 32 * kCells * sizeof(double);
-  if (kSmem > kDefaultSmem && cudaFuncSetAttribute(eval_jacobian_kernel<kCells>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem) != cudaSuccess)
-    return MKPP_ERROR_DEVICE;
-  eval_jacobian_kernel<kCells><<<dim3(launch_grid(n, 32 * kCells), Mech::NS), kWarps * 32, kSmem, stream>>>(n, conc, ktab,
-                                                                                                           out);
+  constexpr size_t kPartials = (size_t)T::MAX_PARTIALS * 32 * kCells * sizeof(double);
+  constexpr bool kStage = kPartials <= kMaxSmem;
+  constexpr size_t kSmem = kStage ? kPartials : 0;
+  const auto kernel = eval_jacobian_kernel<kCells, kStage>;
+  if (kSmem > kDefaultSmem && !allow_smem(kernel, kSmem)) return MKPP_ERROR_DEVICE;
+  kernel<<<dim3(launch_grid(n, 32 * kCells), Mech::NS), kWarps * 32, kSmem, stream>>>(n, conc, ktab, out);
   return cudaGetLastError() == cudaSuccess ? MKPP_SUCCESS : MKPP_ERROR_DEVICE;
 }
 
@@ -191,11 +211,9 @@ int launch_eval_rates(size_t n, const double* conc, const double* ktab, double* 
     eval_cell_rates_kernel<<<launch_grid(n, 128), 128, 0, stream>>>(n, conc, ktab, out);
     return cudaGetLastError() == cudaSuccess ? MKPP_SUCCESS : MKPP_ERROR_DEVICE;
   }
-  if (kRatesSmem > kDefaultSmem &&
-      cudaFuncSetAttribute(eval_rates_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRatesSmem) !=
-          cudaSuccess)
-    return MKPP_ERROR_DEVICE;
-  eval_rates_kernel<<<launch_grid(n, 32), kRateWarps * 32, kRatesSmem, stream>>>(n, conc, ktab, out);
+  constexpr size_t kSmem = kStageRates ? kRatesSmem : 0;
+  if (kSmem > kDefaultSmem && !allow_smem(eval_rates_kernel, kSmem)) return MKPP_ERROR_DEVICE;
+  eval_rates_kernel<<<launch_grid(n, 32), kRateWarps * 32, kSmem, stream>>>(n, conc, ktab, out);
   return cudaGetLastError() == cudaSuccess ? MKPP_SUCCESS : MKPP_ERROR_DEVICE;
 }
 

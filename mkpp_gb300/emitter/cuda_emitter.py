@@ -1027,12 +1027,20 @@ def _eval_tables(plan) -> str:
     t("// Tables of the evaluation kernels (device constant data).")
     t("namespace eval {")
     factors: list[int] = []
+    # A factor is a species, or (its top bit set) a number.
+    longest = max([sum(pw for _, pw in r.reactants) for r in plan.reactions] + [1]) + 1
+    power = 1 << (15 if max(ns, longest) < 1 << 15 else 31)
+    len_bits = max(4, longest.bit_length())
 
     def product(codes):
         """A product of k_r and these factors: where they start, how many."""
         start = len(factors)
         factors.extend(codes)
-        return start << 4 | len(codes)
+        assert len(codes) < 1 << len_bits and start < 1 << (32 - len_bits), "too many factors for the evaluation tables"
+        return start << len_bits | len(codes)
+
+    def index_type(values):
+        return "unsigned short" if max(values, default=0) < 1 << 16 else "unsigned"
 
     rates = [product([s_ for s_, pw in r.reactants for _ in range(pw)]) for r in plan.reactions]
     columns = {j: [] for j in range(ns)}     # column -> [(reaction, product)]
@@ -1045,7 +1053,7 @@ def _eval_tables(plan) -> str:
                 if x != y:
                     codes += [s2] * pw2
                 elif pw2 > 1:
-                    codes += [0x8000 | pw2] + [s2] * (pw2 - 1)
+                    codes += [power | pw2] + [s2] * (pw2 - 1)
             where[(r.index, s_)] = len(columns[s_])
             columns[s_].append((r.index, product(codes)))
     f_rows = {i: [] for i in range(ns)}
@@ -1073,12 +1081,15 @@ def _eval_tables(plan) -> str:
             j_term += [q for _, q in terms or []]
             j_coef += [_lit(q) for q, _ in terms or []]
     j_ptr.append(len(j_term) << 2)
+    t(f"constexpr int RATES = {len(rates)};         // of a cell")
     t(f"constexpr int MAX_PARTIALS = {max(len(v) for v in columns.values())};   // of one column")
-    for name, ctype, vals in (("factor", "unsigned short", factors), ("rate", "unsigned", rates),
-                              ("f_ptr", "int", f_ptr), ("f_term", "unsigned short", f_term),
+    t(f"constexpr unsigned POWER = {power:#x};  // flag of a factor that is a number")
+    t(f"constexpr int LEN_BITS = {len_bits};     // of a product's code")
+    for name, ctype, vals in (("factor", index_type(factors), factors), ("rate", "unsigned", rates),
+                              ("f_ptr", "int", f_ptr), ("f_term", index_type(f_term), f_term),
                               ("f_coef", "double", f_coef), ("p_ptr", "int", p_ptr),
-                              ("p_rate", "unsigned short", p_rate), ("p_product", "unsigned", p_product),
-                              ("j_ptr", "unsigned", j_ptr), ("j_term", "unsigned short", j_term),
+                              ("p_rate", index_type(p_rate), p_rate), ("p_product", "unsigned", p_product),
+                              ("j_ptr", "unsigned", j_ptr), ("j_term", index_type(j_term), j_term),
                               ("j_coef", "double", j_coef)):
         _c_array(t, ctype, name, vals, per_use=True)
     t("}  // namespace eval")
