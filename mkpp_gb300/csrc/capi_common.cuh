@@ -85,12 +85,14 @@ int launch_coop(const mkpp::LaunchArgs& a, int grid, size_t smem, cudaStream_t s
 // mkpp_capi.cu: calls of at most this many cells run on the cooperative
 // kernels alone.
 int coop_cells();
-// mkpp_coop_sweeps.cu: the differentiation kernels on whole warps.  False where
-// the call goes to the lanes.
+// mkpp_coop_sweeps.cu: the differentiation kernels on whole warps; `next` is
+// room for their work counter.  False where the call goes to the lanes.
 bool sweep_on_warps(size_t cells, bool tangent);
-int launch_checkpoint_coop(const mkpp::LaunchArgs& a, const mkpp::CheckpointArgs& ck, cudaStream_t stream);
-int launch_adjoint_coop(const mkpp::AdjointArgs& a, const mkpp::CheckpointArgs& ck, cudaStream_t stream);
-int launch_tangent_coop(const mkpp::TangentArgs& a, const mkpp::CheckpointArgs& ck, cudaStream_t stream);
+int launch_checkpoint_coop(mkpp::LaunchArgs a, const mkpp::CheckpointArgs& ck, unsigned* next, cudaStream_t stream);
+int launch_adjoint_coop(const mkpp::AdjointArgs& a, const mkpp::CheckpointArgs& ck, unsigned* next,
+                        cudaStream_t stream);
+int launch_tangent_coop(const mkpp::TangentArgs& a, const mkpp::CheckpointArgs& ck, unsigned* next,
+                        cudaStream_t stream);
 // ... and the split form (integrate_split_kernel: whole warps on reserved
 // SMs, the persistent body on the others).
 int launch_split(const mkpp::LaunchArgs& a, double* scratch, int grid, cudaStream_t stream);

@@ -6,12 +6,21 @@ namespace mkpp_tu {
 
 namespace {
 
-// Launches `kernel` with a block of one warp per cell.
+// Launches `kernel` with one warp per block: with a work counter, as many as
+// the cells and the shared memory of the SMs allow, else a block per cell.
 template <class Kernel, class... Args>
-int launch_warps(Kernel kernel, size_t slots, int cells, cudaStream_t stream, const Args&... args) {
+int launch_warps(Kernel kernel, size_t slots, int cells, unsigned* next, cudaStream_t stream, const Args&... args) {
   const size_t smem = slots * sizeof(double);
   if (!allow_smem(kernel, smem)) return MKPP_ERROR_DEVICE;
-  kernel<<<cells, 32, smem, stream>>>(args...);
+  int blocks = cells;
+  if (next) {
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 32, smem) != cudaSuccess || per_sm < 1)
+      return MKPP_ERROR_DEVICE;
+    if (cudaMemsetAsync(next, 0, sizeof(unsigned), stream) != cudaSuccess) return MKPP_ERROR_DEVICE;
+    blocks = std::min(cells, per_sm * sm_count());
+  }
+  kernel<<<blocks, 32, smem, stream>>>(args...);
   return cudaGetLastError() == cudaSuccess ? MKPP_SUCCESS : MKPP_ERROR_DEVICE;
 }
 
@@ -31,16 +40,21 @@ bool sweep_on_warps(size_t cells, bool tangent) {
   return kSlots * sizeof(double) <= kMaxSmem && cells <= most;
 }
 
-int launch_checkpoint_coop(const mkpp::LaunchArgs& a, const mkpp::CheckpointArgs& ck, cudaStream_t stream) {
-  return launch_warps(mkpp::checkpoint_coop_kernel<Mech>, Mech::WARP_SLOTS, a.ncells, stream, a, ck);
+int launch_checkpoint_coop(mkpp::LaunchArgs a, const mkpp::CheckpointArgs& ck, unsigned* next, cudaStream_t stream) {
+  if (!mkpp::StoreN<Mech::NSLOTS>::kTile) next = nullptr;
+  a.coop_next = next;
+  return launch_warps(mkpp::checkpoint_coop_kernel<Mech>, Mech::WARP_SLOTS, a.ncells, next, stream, a, ck);
 }
 
-int launch_adjoint_coop(const mkpp::AdjointArgs& a, const mkpp::CheckpointArgs& ck, cudaStream_t stream) {
-  return launch_warps(mkpp::adjoint_coop_kernel<Mech>, Mech::ADJ_COOP_SLOTS, a.ncells, stream, a, ck);
+int launch_adjoint_coop(const mkpp::AdjointArgs& a, const mkpp::CheckpointArgs& ck, unsigned* next,
+                        cudaStream_t stream) {
+  if (!mkpp::StoreN<Mech::NSLOTS_ADJ>::kTile) next = nullptr;
+  return launch_warps(mkpp::adjoint_coop_kernel<Mech>, Mech::ADJ_COOP_SLOTS, a.ncells, next, stream, a, ck, next);
 }
 
-int launch_tangent_coop(const mkpp::TangentArgs& a, const mkpp::CheckpointArgs& ck, cudaStream_t stream) {
-  return launch_warps(mkpp::tangent_coop_kernel<Mech>, Mech::TLM_COOP_SLOTS, a.ncells, stream, a, ck);
+int launch_tangent_coop(const mkpp::TangentArgs& a, const mkpp::CheckpointArgs& ck, unsigned* next,
+                        cudaStream_t stream) {
+  return launch_warps(mkpp::tangent_coop_kernel<Mech>, Mech::TLM_COOP_SLOTS, a.ncells, next, stream, a, ck, next);
 }
 
 }  // namespace mkpp_tu
