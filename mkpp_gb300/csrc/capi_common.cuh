@@ -87,7 +87,8 @@ int launch_coop(const mkpp::LaunchArgs& a, int grid, size_t smem, cudaStream_t s
 int coop_cells();
 // mkpp_coop_sweeps.cu: the differentiation kernels on whole warps; `next` is
 // room for their work counter.  False where the call goes to the lanes.
-bool sweep_on_warps(size_t cells, bool tangent);
+enum class Sweep { kForward, kAdjoint, kTangent };
+bool sweep_on_warps(size_t cells, Sweep sweep);
 int launch_checkpoint_coop(mkpp::LaunchArgs a, const mkpp::CheckpointArgs& ck, unsigned* next, cudaStream_t stream);
 int launch_adjoint_coop(const mkpp::AdjointArgs& a, const mkpp::CheckpointArgs& ck, unsigned* next,
                         cudaStream_t stream);

@@ -28,16 +28,30 @@ constexpr size_t kSlots = std::max(std::max(Mech::WARP_SLOTS, Mech::ADJ_COOP_SLO
 
 }  // namespace
 
-// Up to as many cells as a plain integrate; register stores longer: small_strato's
-// gradient 6.3 against 6.6 ms for 2000 cells, 11.3 against 9.7 for 4325, and its
-// tangent, whose lanes walk a program on the global tile, 9.6 ms for 4325 cells
-// and 13.5 for 8000 against 14 on lanes.
-bool sweep_on_warps(size_t cells, bool tangent) {
-  constexpr size_t kRegister = Mech::NLU > 20 ? 2000 : 300, kTangent = Mech::NLU > 20 ? 8000 : 300;
-  const size_t most = coop_cells() == 0 ? 0
-                      : StoreInfo::kTile ? (size_t)coop_cells()
-                                         : (tangent ? kTangent : kRegister);
-  return kSlots * sizeof(double) <= kMaxSmem && cells <= most;
+// Up to this many cells; the lanes' time hardly depends on their number until
+// they fill the SMs.  Warps against lanes:
+//   SAPRC99's gradient: 2048 cells 88 against 484 ms, 10000 cells 165 against 485;
+//   saprc99_mini's: 4000 cells 4.3 against 10.7 ms, 8000 cells 5.2 against 10.3;
+//   register stores: small_strato's gradient 6.3 against 9.5 ms for 2000 cells,
+//   11.3 against 9.7 for 4325, its tangent, whose lanes walk a program on the
+//   global tile, 9.3 against 14.5 ms for 4000 cells and 13.6 against 14.5 for
+//   8000; Chapman's gradient 1.35 against 1.57 ms for 300 cells;
+//   TS1, whose lanes walk programs everywhere, nine steps a cell: the forward
+//   134 against 284 ms for 16384 cells, 494 against 639 for 65536; the adjoint,
+//   whose store leaves room for two warps per SM, 271 against 339 ms for 12000
+//   cells, 366 against 370 for 16384, 895 against 606 for 40000; the tangent,
+//   three warps per SM, 250 against 368 ms for 16384, 401 against 403 for 26000,
+//   610 against 601 for 40000, 998 against 843 for 65536.
+bool sweep_on_warps(size_t cells, Sweep sweep) {
+  constexpr bool kLargeRegister = Mech::NLU > 20;
+  size_t most;
+  if (Mech::TABLE_ATTEMPT)
+    most = sweep == Sweep::kForward ? SIZE_MAX : sweep == Sweep::kAdjoint ? 16384 : 26000;
+  else if (StoreInfo::kTile)
+    most = Mech::LU_FMA > 2000 ? 14000 : 10000;
+  else
+    most = !kLargeRegister ? 300 : sweep == Sweep::kTangent ? 8000 : 2000;
+  return coop_cells() > 0 && kSlots * sizeof(double) <= kMaxSmem && cells <= most;
 }
 
 int launch_checkpoint_coop(mkpp::LaunchArgs a, const mkpp::CheckpointArgs& ck, unsigned* next, cudaStream_t stream) {

@@ -47,7 +47,7 @@ int mkpp_gpu_integrate_checkpoint(size_t num_cells, double* conc, const double* 
   mkpp::LaunchArgs a = make_args(num_cells, conc, ktab, 1, dt, seed, max_attempts, status, accepted, rejected);
   mkpp::CheckpointArgs ck{ckpt_cap, ckpt_y, ckpt_h, ckpt_n};
   // The workspace's first 256 bytes may hold the warps' work counter.
-  if (sweep_on_warps(num_cells, false)) return launch_checkpoint_coop(a, ck, (unsigned*)workspace, (cudaStream_t)stream);
+  if (sweep_on_warps(num_cells, Sweep::kForward)) return launch_checkpoint_coop(a, ck, (unsigned*)workspace, (cudaStream_t)stream);
   double* scratch = (double*)((unsigned char*)workspace + 256);
   return launch_checkpoint(a, ck, scratch, diff_grid(num_cells), (cudaStream_t)stream);
 }
@@ -76,7 +76,7 @@ int mkpp_gpu_adjoint(size_t num_cells, const double* ktab, int ckpt_cap, const d
   mkpp::CheckpointArgs ck{ckpt_cap, const_cast<double*>(ckpt_y), const_cast<double*>(ckpt_h),
                           const_cast<int*>(ckpt_n)};
   // The workspace's first 256 bytes may hold the warps' work counter.
-  if (sweep_on_warps(num_cells, false)) return launch_adjoint_coop(a, ck, (unsigned*)workspace, (cudaStream_t)stream);
+  if (sweep_on_warps(num_cells, Sweep::kAdjoint)) return launch_adjoint_coop(a, ck, (unsigned*)workspace, (cudaStream_t)stream);
   double* scratch = (double*)((unsigned char*)workspace + 256);
   return launch_adjoint(a, ck, scratch, diff_grid(num_cells), (cudaStream_t)stream);
 }
@@ -92,7 +92,7 @@ int mkpp_gpu_tangent(size_t num_cells, const double* ktab, int ckpt_cap, const d
   mkpp::CheckpointArgs ck{ckpt_cap, const_cast<double*>(ckpt_y), const_cast<double*>(ckpt_h),
                           const_cast<int*>(ckpt_n)};
   // The workspace's first 256 bytes may hold the warps' work counter.
-  if (sweep_on_warps(num_cells, true)) return launch_tangent_coop(a, ck, (unsigned*)workspace, (cudaStream_t)stream);
+  if (sweep_on_warps(num_cells, Sweep::kTangent)) return launch_tangent_coop(a, ck, (unsigned*)workspace, (cudaStream_t)stream);
   double* scratch = (double*)((unsigned char*)workspace + 256);
   return launch_tangent(a, ck, scratch, diff_grid(num_cells), (cudaStream_t)stream);
 }
