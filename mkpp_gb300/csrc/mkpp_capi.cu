@@ -147,17 +147,24 @@ struct Tuning {
   int split_sms = 0;
   // Calls of at most this many cells run on the cooperative kernel alone
   // (coop_alone).  A lane needs 1.0 ms for a SAPRC99 attempt and 1.9 ms with
-  // every SM full, a warp 0.17-0.19 ms; with eight warps per SM the warps reach
-  // 5.5 M attempts/s.  One host step: 2500 cells 34 against 163 ms, 8000 cells 55
-  // against 59, 14000 equal, 20000 cells 128 against 115 (lanes whose tail moves
-  // to the warps).  TS1 is always faster there: 36 against 293 ms for 4096
-  // cells.  A mechanism with few operations per attempt spends them on the
-  // parts that every lane of the warp repeats: saprc99_mini wins up to 8192
-  // cells (2500 cells: 1.38 against 3.14 ms; 32768: 8.8 against 7.2 ms), one
-  // whose lanes keep their store in registers a few hundred (small_strato: 72
-  // cells 1.8 against 2.7 ms, 4096 cells 6.1 against 3.5; Chapman: 0.51 against
-  // 0.57 ms, 2.1 against 0.67).
-  int coop_cells = Mech::TABLE_ATTEMPT ? INT32_MAX : Mech::LU_FMA > 2000 ? 14000 : StoreInfo::kTile ? 10000 : 600;
+  // every SM full, a warp 0.17-0.19 ms, and with eight warps per SM the warps
+  // reach 5.5 M attempts/s; a mechanism with few operations per attempt spends
+  // them on the parts that every lane of the warp repeats.  The integrate call
+  // on warps against lanes (whose tail moves to the warps), 152 SMs, ms:
+  //   SAPRC99       2500 cells 31 / 44, 8000 58 / 62, 14000 84 / 80, 20000 114 /
+  //                 98; four host steps 333 cells 34 / 62, 8000 114 / 125,
+  //                 14000 174 / 182, 20000 244 / 235
+  //   TS1           100 cells 4.4 / 113, 4096 31 / 175, 40000 296 / 430, 262144
+  //                 1936 / 2189
+  //   saprc99_mini  1000 cells 1.04 / 1.67, 4000 1.46 / 1.87, 8000 1.98 / 1.87,
+  //                 10000 2.20 / 1.92, 32768 6.1 / 3.2; four host steps 4000
+  //                 cells 3.5 / 5.6, 10000 6.1 / 6.0
+  //   small_strato  72 cells 1.55 / 1.74, 300 1.80 / 2.57, 600 1.91 / 2.70, 2000
+  //                 2.54 / 2.71, 4096 4.4 / 2.9
+  //   Chapman       72 cells 0.40 / 0.48, 300 0.42 / 0.50, 600 0.42 / 0.50, 1000
+  //                 0.47 / 0.51, 2000 0.74 / 0.52
+  // Register stores share one line, where the warps of both win.
+  int coop_cells = Mech::TABLE_ATTEMPT ? INT32_MAX : Mech::LU_FMA > 2000 ? 14000 : StoreInfo::kTile ? 8000 : 600;
 };
 
 Tuning& tuning() {
