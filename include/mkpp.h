@@ -104,10 +104,11 @@ int mkpp_set_max_attempts(mkpp_handle_t handle, int max_attempts);
 int mkpp_get_cell_stats(mkpp_handle_t handle, int* status, int* accepted, int* rejected);
 /* Cost ordering (default on): each mkpp_integrate hands out first the cells
  * that needed the most attempts in the previous call on this handle, so the
- * slowest cells start first and the call's tail shrinks.  Results do not
- * depend on it (cells are independent); it reads back num_cells x 2 ints per
- * call and sends the order (num_cells ints).  enable 0 turns it off and
- * forgets the counts. */
+ * slowest cells start first and the call's tail shrinks.  Where all cells of
+ * the handle start at once no order could help, and none is made.  Results do
+ * not depend on it (cells are independent); an ordered call reads back
+ * num_cells x 2 ints and sends the order (num_cells ints).  enable 0 turns it
+ * off and forgets the counts. */
 int mkpp_set_cost_order(mkpp_handle_t handle, int enable);
 /* Step-size carry-over (default off; no reference entry: the reference
  * restarts every integrate() at dt * initial_step_seed and lists carried
@@ -148,15 +149,27 @@ size_t mkpp_gpu_workspace_bytes(size_t num_cells);
  * step of a launch (a launch over S steps: defer_after * S in all) after which
  * the persistent kernel hands a cell to the warp-cooperative kernel (0: never,
  * -1 keeps the current value; default 3000, environment MKPP_DEFER_AFTER).
- * Results do not depend on it: a handed-off cell ends bit-identical. */
+ * Results do not depend on it: a handed-off cell ends bit-identical.
+ *
+ * A persistent call of few cells runs on the warp-cooperative kernel from the
+ * start, a warp per cell, and has no cells to hand off: up to 14000 cells of
+ * SAPRC99's size, a few hundred to 8000 of smaller mechanisms, any number of
+ * TS1's (csrc/mkpp_capi.cu has the rule).  The environment's MKPP_COOP_CELLS
+ * is another such number of cells, 0 for none; 0 also keeps every
+ * differentiated call on lanes, whose limits are otherwise their own.  Calls
+ * stay on the persistent kernel where defer_after is 0, register_variant 4,
+ * blocks_per_sm set, or a split launch asked for. */
 int mkpp_set_launch_tuning(int register_variant, int blocks_per_sm, int defer_after);
 
 /* Process-wide tail parking of the persistent integrate kernel (default 16
  * attempts, 0: off; environment MKPP_TAIL_AFTER).  Once every cell of a launch has been
- * handed out and no more cells are still on lanes than the warp-cooperative
- * kernel runs at once, a cell with at least min_attempts attempts is parked
- * for that kernel, which takes a warp per cell.  The last, slowest cells of a
- * call then finish faster.  Results do not depend on it: a parked cell ends
+ * handed out and few cells are still on lanes, a cell with at least
+ * min_attempts attempts is parked for the warp-cooperative kernel, which takes
+ * a warp per cell.  Few: 16 for each warp that this kernel runs at once where
+ * the LU has more than 2000 multiply-adds (SAPRC99, TS1), 2 for each where it
+ * has fewer, and one per SM where lanes keep a cell's store in registers
+ * (Chapman, small_strato).  The last, slowest cells of a call then finish
+ * faster.  Results do not depend on it: a parked cell ends
  * bit-identical.  Applies to the 255-register variant. */
 int mkpp_set_tail_parking(int min_attempts);
 /* Split launch (process-wide, default off; no reference counterpart): when
@@ -164,7 +177,7 @@ int mkpp_set_tail_parking(int min_attempts);
  * split_sms SMs integrate its first split_cells cells, each on a whole warp
  * (the warp-cooperative attempt), while the other SMs run the persistent
  * kernel's body over the rest of the order, in the same launch.  A warp on
- * an SM that runs no lanes finishes an attempt of one cell about 3x sooner
+ * an SM that runs no lanes finishes an attempt of one cell about 5x sooner
  * than a lane, so the few most expensive cells, which otherwise set the end
  * of the launch, finish earlier.  Results are bit-identical.  Applies to the
  * 255-register variant without tail parking.  Give the cells in cost order
@@ -233,7 +246,8 @@ int mkpp_gpu_evaluate_jacobian(size_t num_cells, const double* conc, const doubl
  * full discrete adjoint of the accepted steps, with the Jacobian's
  * dependence on the state and on the rate constants) ------------------- */
 #define MKPP_CELL_ERR_CHECKPOINT_OVERFLOW 5
-/* Workspace of the three calls below (per-thread scratch, 256-byte aligned). */
+/* Workspace of the three calls below (work counter and per-thread scratch,
+ * 256-byte aligned).  Calls that overlap on the GPU need one each. */
 size_t mkpp_gpu_adjoint_workspace_bytes(size_t num_cells);
 /* One integrate() call over dt (same controller and arithmetic as the plain
  * form) that records, at every accepted step s < ckpt_cap, the state before
@@ -262,7 +276,8 @@ int mkpp_gpu_adjoint(size_t num_cells, const double* ktab, int ckpt_cap, const d
  * integrate_tlm.j2:32-215, a frozen-Jacobian tangent in the state alone;
  * this one is the exact tangent of the accepted steps, the transpose of
  * mkpp_gpu_adjoint, and also carries a direction in the rate constants) --- */
-/* Workspace of mkpp_gpu_tangent (per-thread scratch, 256-byte aligned). */
+/* Workspace of mkpp_gpu_tangent (work counter and per-thread scratch, 256-byte
+ * aligned); calls that overlap on the GPU need one each. */
 size_t mkpp_gpu_tangent_workspace_bytes(size_t num_cells);
 /* Given the checkpoints of mkpp_gpu_integrate_checkpoint, a direction
  * delta_conc0 in the starting state ([species][cells]; fixed species

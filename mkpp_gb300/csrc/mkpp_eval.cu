@@ -6,9 +6,9 @@
 //
 // Both are bound by memory: the Jacobian is NS^2 values per cell written once.
 // A block takes 32 cells, one per lane (64 for the Jacobian), and its warps
-// share their rates (or one column's partial derivatives) in shared memory and divide the rows, so
-// that every output row is one coalesced store per warp and a small call
-// still has blocks for all SMs.  A thread per cell, which zero-filled the
+// share their rates (or one column's partial derivatives) in shared memory and
+// divide the rows, so that every output row is one coalesced store per warp and
+// a small call still has blocks for all SMs.  A thread per cell, which zero-filled the
 // matrix, wrote W and flipped its sign through tables of slot positions on the
 // stack, took 92.8 ms for SAPRC99's 20000 cells (1.08 GB); this takes 0.23 ms.
 // TS1, 1001 cells: 4.5 -> 0.11 ms, the tendencies 3.1 -> 0.06 ms.
@@ -223,7 +223,7 @@ int launch_eval_jacobian(size_t n, const double* conc, const double* ktab, doubl
     return cudaGetLastError() == cudaSuccess ? MKPP_SUCCESS : MKPP_ERROR_DEVICE;
   }
   // Two cells per lane halve the table reads of an output (SAPRC99, 20000
-  // cells: 279 -> 243 us), but need twice the shared memory (TS1, 30 KB for a
+  // cells: 279 -> 234 us), but need twice the shared memory (TS1, 30 KB for a
   // column of one cell a lane: 107 -> 137 us for 1001 cells) and enough blocks
   // (100 SAPRC99 cells: 17 us, 23 with two).
   if (T::MAX_PARTIALS <= 96 && n >= 2048) return launch_jacobian<2>(n, conc, ktab, out, stream);

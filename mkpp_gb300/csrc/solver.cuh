@@ -7,9 +7,9 @@
 //   ktab   [NR][ncells]   rate constants, written by rate_constant_kernel
 //   temp/rho/rh/clw [ncells]
 //
-// One thread owns one cell.  The per-cell controller reproduces
-// SolverKernels::integrate (src/mkpp/templates/solver_variants/integrate.j2:71-84,
-// 324-379): dt0 = dt_total * seed, h_min = dt_total * 1e-15,
+// One thread owns one cell, or in the cooperative forms one warp.  The per-cell
+// controller reproduces SolverKernels::integrate
+// (src/mkpp/templates/solver_variants/integrate.j2:71-84, 324-379): dt0 = dt_total * seed, h_min = dt_total * 1e-15,
 // dt = min(dt, dt_total - t), factor clamp [0.2, 6], no growth right after a
 // rejection, tenfold cut after two consecutive rejections.  Unlike the
 // reference, every integrate() call is bounded by max_attempts; a cell that

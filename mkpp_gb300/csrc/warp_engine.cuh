@@ -67,8 +67,9 @@ struct StepWords<WideWord> {
 // uses takes 108, so a step is an FMA, the store of its result and the loads of
 // the next operands.  Measured on SAPRC99's 2296 steps, up to four warps on an SM:
 // 164 cycles a step in the LU (5 of them bank conflicts, some 28 the steps with
-// reciprocals, by their number) and 111-120 in the solves, and with eight 209 and 143-150 (the FP64 pipe's
-// bound there is 152); 172 and 204 on average with a vote for pivots in every
+// reciprocals, by their number) and 111-120 in the solves, and with eight 209 and
+// 143-150 (the FP64 pipe's bound there is 138: 2482 instructions an attempt, two
+// warps to a pipe); 172 and 204 on average with a vote for pivots in every
 // step, operand loads under branches and the words of a step each waited for
 // alone.
 template <int kPivotEvery>

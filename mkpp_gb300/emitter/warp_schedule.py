@@ -32,7 +32,7 @@ steps of at most 32 for the device loop of csrc/warp_engine.cuh, which stores a
 step's results during the next step and loads operands one step ahead: a value
 is readable from its slot two steps after the operation that makes it, and one
 step after it by the same lane alone, from the register that holds the lane's
-previous result ("forwarded").  SAPRC99's attempt takes 2288 steps, of which
+previous result ("forwarded").  SAPRC99's attempt takes 2296 steps, of which
 1722 are the dependence chain of its three solves, whose row sums keep a fixed
 order.
 
